@@ -104,6 +104,11 @@ template <typename T> struct Vec2;
 template <> struct Vec2<double> { typedef double2 type; };
 template <> struct Vec2<float>  { typedef float2 type; };
 
+// Elements of a twiddle table: complex values, for FP64 (cos, sin) in fixed
+// point (fft_fixed.cuh).
+template <typename T> struct TwVec { typedef typename Vec2<T>::type type; };
+template <> struct TwVec<double> { typedef int4 type; };
+
 template <typename T>
 __device__ __forceinline__ C<T> ldc(const typename Vec2<T>::type* p) {
     typename Vec2<T>::type v = *p;

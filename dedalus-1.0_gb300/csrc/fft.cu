@@ -28,7 +28,7 @@ static bool is_supported_len(int64_t n) {
 // exp(-2 pi i m / L) for m < L, from the first octant by symmetry so that the
 // quadrant points are exact.  Long double keeps the rounding to double
 // essentially correct.
-static void make_twiddles(int L, std::vector<double>& re, std::vector<double>& im) {
+static void make_twiddles(int L, std::vector<long double>& re, std::vector<long double>& im) {
     re.resize(L);
     im.resize(L);
     const long double two_pi = 6.283185307179586476925286766559005768L;
@@ -51,37 +51,54 @@ static void make_twiddles(int L, std::vector<double>& re, std::vector<double>& i
             case 2: C = -c; S = -s; break;
             default: C = s; S = -c; break;
         }
-        re[m] = (double)C;
-        im[m] = (double)(-S);
+        re[m] = C;
+        im[m] = -S;
     }
 }
 
-// The FP64 and FP32 tables hold W_L^m = g (1 + i t) as (g, t) for the
-// fused multiply-add butterflies (fft_engine.cuh): g = Re W, t = Im W / Re W
-// (an IEEE division of the rounded parts, so every host gives the same
-// table); where Re W = 0 the pair is (2^-60, Im W 2^60), exact powers of two
-// whose product is Im W.  The double-float table keeps (cos, sin).
-static int upload_twiddles(int L, double2** d64, float2** d32, float4** ddf) {
-    std::vector<double> re, im;
-    make_twiddles(L, re, im);
-    std::vector<double2> h64(L);
+// cos, sin of one angle as (h, l) with h 2^32 + l = 2^62 cos, both signed halves
+// (l never -2^31: the transforms negate it).
+static int4 fixed_twiddle(long double c, long double s) {
+    auto split = [](long double x, int& h, int& l) {
+        int64_t w = llroundl(ldexpl(x, 62));
+        if ((uint32_t)w == 0x80000000u) w += 1;
+        l = (int32_t)(uint32_t)w;
+        h = (int32_t)((w - l) >> 32);
+    };
+    int4 t;
+    split(c, t.x, t.y);
+    split(s, t.z, t.w);
+    return t;
+}
+
+// The FP64 table holds (cos, sin) of 2 pi m / L in fixed point (fft_fixed.cuh).
+// The FP32 table holds W_L^m = g (1 + i t) as (g, t) for the fused
+// multiply-add butterflies (fft_engine.cuh): g = Re W, t = Im W / Re W (an IEEE
+// division of the rounded parts, so every host gives the same table); where
+// Re W = 0 the pair is (2^-60, Im W 2^60), exact powers of two whose product is
+// Im W.  The double-float table keeps (cos, sin).
+static int upload_twiddles(int L, int4** d64, float2** d32, float4** ddf) {
+    std::vector<long double> rel, iml;
+    make_twiddles(L, rel, iml);
+    const std::vector<double> re(rel.begin(), rel.end()), im(iml.begin(), iml.end());
+    std::vector<int4> h64(L);
     std::vector<float2> h32(L);
     std::vector<float4> hdf(L);
     const double tiny = ldexp(1.0, -60), huge = ldexp(1.0, 60);
     for (int m = 0; m < L; m++) {
+        h64[m] = fixed_twiddle(rel[m], -iml[m]);
         double g, t;
         if (re[m] == 0.0) { g = tiny; t = im[m] * huge; }
         else { g = re[m]; t = im[m] / re[m]; }
-        h64[m] = make_double2(g, t);
         const float g32 = (float)g;
         h32[m] = make_float2(g32, re[m] == 0.0 ? (float)t : (float)(im[m] / (double)g32));
         const df64 a(re[m]), b(im[m]);
         hdf[m] = make_float4(a.hi, a.lo, b.hi, b.lo);
     }
-    DD_CUDA(cudaMalloc((void**)d64, sizeof(double2) * L));
+    DD_CUDA(cudaMalloc((void**)d64, sizeof(int4) * L));
     DD_CUDA(cudaMalloc((void**)d32, sizeof(float2) * L));
     DD_CUDA(cudaMalloc((void**)ddf, sizeof(float4) * L));
-    DD_CUDA(cudaMemcpy(*d64, h64.data(), sizeof(double2) * L, cudaMemcpyHostToDevice));
+    DD_CUDA(cudaMemcpy(*d64, h64.data(), sizeof(int4) * L, cudaMemcpyHostToDevice));
     DD_CUDA(cudaMemcpy(*d32, h32.data(), sizeof(float2) * L, cudaMemcpyHostToDevice));
     DD_CUDA(cudaMemcpy(*ddf, hdf.data(), sizeof(float4) * L, cudaMemcpyHostToDevice));
     return DD_OK;

@@ -13,7 +13,9 @@
 // come from a per-length table W_L^m = exp(-2 pi i m / L) staged in shared
 // memory (conjugated for the inverse transform).
 //
-// FP64 and FP32 butterflies are written for fused multiply-add hardware
+// FP32 and double-float transforms run here; FP64 ones run in block fixed point
+// on the integer pipes (fft_fixed.cuh) with the schedules of this file's form.
+// FP32 butterflies are written for fused multiply-add hardware
 // (Linzer and Feig, "Implementation of efficient FFT algorithms on fused
 // multiply-add architectures", IEEE Trans. Signal Processing 41(1), 1993):
 // a twiddle is stored as (g, t) with W = g (1 + i t), t = Im W / Re W, so
@@ -144,10 +146,8 @@ __device__ __forceinline__ void dft(C<T>* v) {
 
 // --------------------------------------------------- FMA (Linzer-Feig) butterflies
 template <typename T> struct IsLF { static constexpr bool value = false; };
-template <> struct IsLF<double> { static constexpr bool value = true; };
 template <> struct IsLF<float> { static constexpr bool value = true; };
 
-__device__ __forceinline__ double fmx(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fmx(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 // tan(pi/8) and tan(3 pi/8) = sqrt(2) -+ 1 (correctly rounded decimal expansions)
@@ -420,8 +420,7 @@ struct Pencil {
 };
 
 // One Stockham pass of radix R with current sub-transform length NS.  tw is
-// the staged twiddle table: (g, t) pairs for FP64 / FP32, (cos, sin) for
-// double-float.
+// the staged twiddle table: (g, t) pairs for FP32, (cos, sin) for double-float.
 template <typename T, class S, int R, int NS, bool INV, unsigned ZIN = 0u, unsigned ZOUT = 0u>
 __device__ __forceinline__ void stockham_pass(C<T>* tile, const C<T>* tw, int p, int jt) {
     constexpr int L = S::L, TPP = S::TPP;
@@ -475,7 +474,7 @@ __device__ __forceinline__ void stockham_pass(C<T>* tile, const C<T>* tw, int p,
 // threads of the block (all of them must reach the barriers: threads beyond
 // S::NT call with active = false).  The caller synchronises before (tile
 // filled); this returns synchronised with the result in natural order.
-// PRUNE (FP64 / FP32 only, with at least two passes): the pencils follow the
+// PRUNE (FP32 only, with at least two passes): the pencils follow the
 // 2/3 rule, so an inverse transform's first pass skips the inputs in the
 // removed band (they are zero) and a forward transform's last pass skips the
 // outputs in it (the caller never reads them; those tile entries are left

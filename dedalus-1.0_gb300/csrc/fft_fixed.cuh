@@ -1,0 +1,629 @@
+// FP64 pencil transforms on the integer pipes.
+//
+// GB300 issues 2 FP64 operations per clock and SM against 64 integer
+// multiply-adds (32 x 32 + 64 bits) and 64 to 128 integer additions, and
+// its FP64 <-> integer conversion instructions run at the FP64 rate too.  A
+// transform is linear and its growth is known, so a pencil of doubles is
+// transformed as block fixed point: one power-of-two scale per pencil, 64-bit
+// integer values, FP64 bit patterns taken apart and put together with integer
+// instructions.  Additions are exact; a twiddle product rounds once.
+//
+// Scale.  m = largest |re|, |im| of the pencil, read off the high words.  The
+// first pass (radix R1) is bounded by R1 sqrt(2) m, and the scale is the
+// power of two that puts this bound at 2^62.  Every later pass looks at the
+// largest value that the pass before it wrote and divides (or multiplies) by
+// the power of two that keeps its own bound at 2^62; the twiddle product's
+// final shift does the division.  So the words stay filled whether the pencil
+// is a few large modes or noise, the rounding errors of the earlier passes
+// shrink with each division, and the result, rounded to FP64 once at the end,
+// is closer to the exact transform than an FP64 FFT's.
+//
+// Conversions.  On the way in, real parts go through the conversion instruction
+// (FP64 pipe) and imaginary parts are taken apart with integer instructions, so
+// that both pipes work; on the way out everything is integer.
+//
+// Values below 2^-62 of the bound vanish, as they do in an FP64 sum with the
+// larger ones.  A pencil whose largest value is outside 2^-895 .. 2^49 is
+// scaled by 2^512 or 2^-975 on the way in and back on the way out.  One that holds a NaN or an
+// infinity gives NaN everywhere.
+#pragma once
+#include <type_traits>
+
+#include "fft_engine.cuh"
+
+namespace dd {
+
+typedef long long fx;      // one fixed-point value
+
+// --------------------------------------------------- scales
+// 1 - largest |x| high word of a pencil (0 = all zero) to its bound: every
+// component is below 2^(e2 - 1022.5), a pair's modulus below 2^(e2 - 1022).
+// rare: 0, or 1 (times 2^512 on the way in), 2 (times 2^-975), 3 (not finite).
+struct FxScale {
+    int e2, rare;
+};
+
+__host__ __device__ __forceinline__ FxScale fx_scale(unsigned m) {
+    FxScale s;
+    // exponent of sqrt(2) (m + 1): carries where the 20 mantissa bits exceed sqrt(2) - 1
+    s.e2 = (int)((m + 614242u) >> 20);
+    s.rare = 0;
+    if (m == 0u) s.e2 = 1023;
+    else if (m >= 0x7ff00000u) { s.rare = 3; s.e2 = 1023; }
+    else if (s.e2 < 128) { s.rare = 1; s.e2 = (s.e2 > 1 ? s.e2 : 1) + 512; }
+    else if (s.e2 > 1072) { s.rare = 2; s.e2 -= 975; }
+    return s;
+}
+__host__ __device__ __forceinline__ double fx_pre(int rare) {
+    return rare == 1 ? 0x1p512 : rare == 2 ? 0x1p-975 : 1.0;
+}
+__device__ __forceinline__ double fx_post(int rare) {
+    return rare == 1 ? 0x1p-512 : rare == 2 ? 0x1p975 : __longlong_as_double(0x7ff8000000000000ll);
+}
+
+// v[i] *= f behind a branch: FP64 instructions take 64 clocks of their pipe
+// per warp even where a predicate turns them off, and a branch around each
+// single one becomes such a predicate.
+template <int N>
+__device__ __forceinline__ void fx_scale_all(C<double>* v, double f) {
+#pragma unroll
+    for (int i = 0; i < N; i++) { v[i].x *= f; v[i].y *= f; }
+}
+
+// --------------------------------------------------- conversions
+__device__ __forceinline__ unsigned fx_absword(double x) { return (unsigned)__double2hiint(x) << 1; }
+__device__ __forceinline__ unsigned fx_max(unsigned h, C<double> v) {   // words shifted left by one: no mask for the sign
+    return max(h, max(fx_absword(v.x), fx_absword(v.y)));
+}
+
+// x times 2^(1085 - K), for |x| below that scale's 2^62 (K - the biased
+// exponent of x is at least 2, and K <= 1085).  fx_in takes the bit pattern
+// apart (truncating), fx_in64 adds to the exponent and converts (rounding).
+__device__ __forceinline__ fx fx_in(double x, int K) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int k = min(K - (int)((hi << 1) >> 21), 63);
+    const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+    const unsigned H = __funnelshift_l(lo, mh, 10), L = lo << 10;     // mantissa in bits 62 .. 10
+    const unsigned rl = __funnelshift_rc(__funnelshift_rc(L, H, k), 0u, max(k - 32, 0));
+    const unsigned rh = __funnelshift_rc(H, 0u, k);
+    const fx v = (fx)(((unsigned long long)rh << 32) | rl);
+    return (int)hi < 0 ? -v : v;
+}
+__device__ __forceinline__ fx fx_in64(double x, int K) {
+    return __double2ll_rn(__hiloint2double(__double2hiint(x) + ((1085 - K) << 20), __double2loint(x)));
+}
+__device__ __forceinline__ C<fx> fx_in(C<double> v, int K) { return mk<fx>(fx_in64(v.x, K), fx_in(v.y, K)); }
+
+// The double nearest to x 2^(eb - 1085): x in sign and magnitude, normalised,
+// the exponent added to the high word (the leading one adds the last 1 of it).
+// (The two FP64 additions that would join the words as mantissas of two doubles
+// take longer than these instructions in the x pass and as long elsewhere.)
+__device__ __forceinline__ double fx_out(fx x, int eb) {
+    const int sgn = (int)(x >> 32);
+    const unsigned long long a = (unsigned long long)(sgn < 0 ? -x : x);
+    const unsigned hi = (unsigned)(a >> 32), lo = (unsigned)a;
+    int n = __clz((int)hi);
+    unsigned H = __funnelshift_lc(lo, hi, n), L = __funnelshift_lc(0u, lo, n);
+    if (n == 32) {                             // below 2^32
+        const int n2 = __clz((int)H);
+        if (n2 == 32) return 0.0;
+        H <<= n2;
+        n += n2;
+    }
+    const unsigned long long r = (((unsigned long long)H << 32) | L) >> 11;
+    const unsigned long long v = r + ((L >> 10) & 1u) + ((unsigned long long)(unsigned)((eb - n) << 20) << 32);
+    return __hiloint2double((int)((unsigned)(v >> 32) | ((unsigned)sgn & 0x80000000u)), (int)(unsigned)v);
+}
+__device__ __forceinline__ C<double> fx_out(C<fx> v, int eb) { return mk<double>(fx_out(v.x, eb), fx_out(v.y, eb)); }
+
+// --------------------------------------------------- products
+__device__ __forceinline__ fx fx_mad(int a, int b, fx c) { return (fx)a * b + c; }
+
+struct FxHL {
+    int h, l;              // value = h 2^32 + l, both signed
+};
+__device__ __forceinline__ FxHL fx_split(fx a) {
+    FxHL s;
+    s.l = (int)a;
+    s.h = (int)(a >> 32) + (int)((unsigned)s.l >> 31);
+    return s;
+}
+
+__device__ __forceinline__ fx fx_shr(fx a, int n) {       // 0 <= n < 32
+    const unsigned lo = (unsigned)a;
+    const int hi = (int)(a >> 32);
+    return (fx)(((unsigned long long)(unsigned)(hi >> n) << 32) | __funnelshift_r(lo, (unsigned)hi, n));
+}
+__device__ __forceinline__ fx fx_shl(fx a, int n) {       // 0 <= n < 32
+    const unsigned lo = (unsigned)a, hi = (unsigned)(a >> 32);
+    return (fx)(((unsigned long long)__funnelshift_l(lo, hi, n) << 32) | (lo << n));
+}
+
+// a (c + i s) / 2^(2 + n) for a twiddle c + i s = (w.x 2^32 + w.y + i (w.z 2^32 + w.w)) 2^-62
+// (signed halves), half = 2^(31 + n): rounded to nearest up to the product of
+// the low halves (below one unit before the division).  |a| < 2^62, n <= 2.
+__device__ __forceinline__ C<fx> fx_twiddle(C<fx> a, int4 w, int n, fx half) {
+    const FxHL x = fx_split(a.x), y = fx_split(a.y);
+    fx re = fx_mad(x.h, w.y, half), im = fx_mad(x.h, w.w, half);
+    re = fx_mad(x.l, w.x, re);
+    im = fx_mad(x.l, w.z, im);
+    re = fx_mad(y.h, -w.w, re);
+    im = fx_mad(y.h, w.y, im);
+    re = fx_mad(y.l, -w.z, re) >> 32;
+    im = fx_mad(y.l, w.x, im) >> 32;
+    re = fx_mad(x.h, w.x, re);
+    im = fx_mad(x.h, w.z, im);
+    re = fx_mad(y.h, -w.z, re);
+    im = fx_mad(y.h, w.x, im);
+    return mk<fx>(fx_shr(re, n), fx_shr(im, n));
+}
+
+// a times the constant (CH 2^32 + CL) 2^-63, rounded to nearest; |a| < 2^62.
+__device__ __forceinline__ fx fx_mul63(fx a, int ch, int cl) {
+    const FxHL x = fx_split(a);
+    const fx t = fx_mad(x.l, ch, fx_mad(x.h, cl, 1ll << 30)) >> 31;
+    return fx_mad(2 * x.h, ch, t);
+}
+
+// sqrt(1/2) and sqrt(3)/2 in units of 2^-63
+#define DD_FX_R2H 1518500250
+#define DD_FX_R2L (-51432894)
+#define DD_FX_S3H 1859775393
+#define DD_FX_S3L 1630710223
+// cos and sin of pi/8 in units of 2^-62
+#define DD_FX_C8H 992008094
+#define DD_FX_C8L 1696238673
+#define DD_FX_S8H 410903207
+#define DD_FX_S8L (-1364630830)
+
+// a W_16^M (forward) or its conjugate (inverse), M a compile-time constant;
+// |a| < 2^60 (odd M) or 2^61.
+template <int M, bool INV>
+__device__ __forceinline__ C<fx> fx_rot16(C<fx> a) {
+    constexpr int m = M % 16;
+    if constexpr (m == 0) {
+        return a;
+    } else if constexpr (m == 4) {
+        return mul_mi<INV>(a);
+    } else if constexpr (m == 2) {             // (1 -+ i) / sqrt 2
+        const fx p = fx_mul63(a.x + a.y, DD_FX_R2H, DD_FX_R2L), d = fx_mul63(a.y - a.x, DD_FX_R2H, DD_FX_R2L);
+        return INV ? mk<fx>(-d, p) : mk<fx>(p, d);
+    } else if constexpr (m == 6) {             // (-1 -+ i) / sqrt 2
+        const fx p = fx_mul63(a.x + a.y, DD_FX_R2H, DD_FX_R2L), d = fx_mul63(a.y - a.x, DD_FX_R2H, DD_FX_R2L);
+        return INV ? mk<fx>(-p, -d) : mk<fx>(d, -p);
+    } else {
+        static_assert(m == 1 || m == 3 || m == 9, "unused rotation");
+        // 4 a.h fits 32 bits
+        constexpr bool swap = m == 3;
+        constexpr int sg = m == 9 ? -1 : 1;    // W^9 = -W^1
+        constexpr int ch = sg * (swap ? DD_FX_S8H : DD_FX_C8H), cl = sg * (swap ? DD_FX_S8L : DD_FX_C8L);
+        constexpr int s0h = sg * (swap ? DD_FX_C8H : DD_FX_S8H), s0l = sg * (swap ? DD_FX_C8L : DD_FX_S8L);
+        constexpr int sh = INV ? s0h : -s0h, sl = INV ? s0l : -s0l;
+        const FxHL x = fx_split(a.x), y = fx_split(a.y);
+        const fx half = 1ll << 29;
+        fx re = fx_mad(x.l, ch, fx_mad(x.h, cl, half)), im = fx_mad(x.l, sh, fx_mad(x.h, sl, half));
+        re = fx_mad(y.l, -sh, fx_mad(y.h, -sl, re)) >> 30;
+        im = fx_mad(y.l, ch, fx_mad(y.h, cl, im)) >> 30;
+        const int x4 = 4 * x.h, y4 = 4 * y.h;
+        re = fx_mad(y4, -sh, fx_mad(x4, ch, re));
+        im = fx_mad(y4, ch, fx_mad(x4, sh, im));
+        return mk<fx>(re, im);
+    }
+}
+
+// --------------------------------------------------- in-register DFTs
+template <int R, bool INV>
+__device__ __forceinline__ void fx_dft(C<fx>* v) {
+    if constexpr (R == 4) {
+        dft4<INV>(v[0], v[1], v[2], v[3]);
+    } else if constexpr (R == 8) {
+        C<fx> e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+        C<fx> o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
+        dft4<INV>(e0, e1, e2, e3);
+        dft4<INV>(o0, o1, o2, o3);
+        o1 = fx_rot16<2, INV>(o1);
+        o2 = fx_rot16<4, INV>(o2);
+        o3 = fx_rot16<6, INV>(o3);
+        v[0] = e0 + o0; v[4] = e0 - o0;
+        v[1] = e1 + o1; v[5] = e1 - o1;
+        v[2] = e2 + o2; v[6] = e2 - o2;
+        v[3] = e3 + o3; v[7] = e3 - o3;
+    } else if constexpr (R == 16) {
+        C<fx> y[4][4];
+#pragma unroll
+        for (int n2 = 0; n2 < 4; n2++) {
+            y[n2][0] = v[n2]; y[n2][1] = v[4 + n2]; y[n2][2] = v[8 + n2]; y[n2][3] = v[12 + n2];
+            dft4<INV>(y[n2][0], y[n2][1], y[n2][2], y[n2][3]);
+        }
+        y[1][1] = fx_rot16<1, INV>(y[1][1]);
+        y[1][2] = fx_rot16<2, INV>(y[1][2]);
+        y[1][3] = fx_rot16<3, INV>(y[1][3]);
+        y[2][1] = fx_rot16<2, INV>(y[2][1]);
+        y[2][2] = fx_rot16<4, INV>(y[2][2]);
+        y[2][3] = fx_rot16<6, INV>(y[2][3]);
+        y[3][1] = fx_rot16<3, INV>(y[3][1]);
+        y[3][2] = fx_rot16<6, INV>(y[3][2]);
+        y[3][3] = fx_rot16<9, INV>(y[3][3]);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; k1++) {
+            C<fx> a0 = y[0][k1], a1 = y[1][k1], a2 = y[2][k1], a3 = y[3][k1];
+            dft4<INV>(a0, a1, a2, a3);
+            v[k1] = a0; v[k1 + 4] = a1; v[k1 + 8] = a2; v[k1 + 12] = a3;
+        }
+    } else {
+        static_assert(R == 3, "unsupported radix");
+        const C<fx> t1 = v[1] + v[2], r = mul_mi<INV>(v[1] - v[2]);
+        const C<fx> m1 = mk<fx>(v[0].x - ((t1.x + 1) >> 1), v[0].y - ((t1.y + 1) >> 1));
+        const C<fx> m2 = mk<fx>(fx_mul63(r.x, DD_FX_S3H, DD_FX_S3L), fx_mul63(r.y, DD_FX_S3H, DD_FX_S3L));
+        v[0] = v[0] + t1;
+        v[1] = m1 + m2;
+        v[2] = m1 - m2;
+    }
+}
+
+// --------------------------------------------------- pencils
+// Default schedules: P pencils of TPP threads, radices, and MB resident blocks
+// per SM (__launch_bounds__).  Radix 8 and 4 passes of one butterfly per thread
+// need 64 registers, so that 1024 threads fit an SM: at 256 points the y passes
+// of a 256^3 step took 248 / 150 us (forward / inverse) against 281 / 178 us for
+// two radix-16 passes (116 registers, 512 threads).  8-pencil tiles keep global
+// accesses at 128 bytes; 4 pencils took 327 / 182 us.  Forward schedules end
+// with radix 8, whose outputs in the removed band are skipped, inverse ones begin
+// with it.
+template <int L> struct FxCfg;
+template <> struct FxCfg<8>   { static constexpr int P = 64, TPP = 1,  MB = 8, R[3] = {8, 1, 1}, RF[3] = {8, 1, 1}; };
+template <> struct FxCfg<16>  { static constexpr int P = 64, TPP = 4,  MB = 4, R[3] = {4, 4, 1}, RF[3] = {4, 4, 1}; };
+template <> struct FxCfg<24>  { static constexpr int P = 64, TPP = 4,  MB = 4, R[3] = {8, 3, 1}, RF[3] = {8, 3, 1}; };
+template <> struct FxCfg<32>  { static constexpr int P = 64, TPP = 4,  MB = 4, R[3] = {8, 4, 1}, RF[3] = {4, 8, 1}; };
+template <> struct FxCfg<48>  { static constexpr int P = 16, TPP = 16, MB = 4, R[3] = {4, 4, 3}, RF[3] = {4, 4, 3}; };
+template <> struct FxCfg<64>  { static constexpr int P = 32, TPP = 8,  MB = 4, R[3] = {8, 8, 1}, RF[3] = {8, 8, 1}; };
+template <> struct FxCfg<96>  { static constexpr int P = 16, TPP = 12, MB = 5, R[3] = {8, 4, 3}, RF[3] = {8, 4, 3}; };
+template <> struct FxCfg<128> { static constexpr int P = 16, TPP = 16, MB = 4, R[3] = {8, 4, 4}, RF[3] = {4, 4, 8}; };
+template <> struct FxCfg<192> { static constexpr int P = 8,  TPP = 24, MB = 5, R[3] = {8, 8, 3}, RF[3] = {8, 8, 3}; };
+template <> struct FxCfg<256> { static constexpr int P = 8,  TPP = 32, MB = 4, R[3] = {8, 8, 4}, RF[3] = {8, 4, 8}; };
+template <> struct FxCfg<512> { static constexpr int P = 8,  TPP = 64, MB = 2, R[3] = {8, 8, 8}, RF[3] = {8, 8, 8}; };
+
+template <int L, bool INV, int P = FxCfg<L>::P, class CC = FxCfg<L>>
+using FxS = Sched<L, P, P * CC::TPP, INV ? CC::R[0] : CC::RF[0], INV ? CC::R[1] : CC::RF[1], INV ? CC::R[2] : CC::RF[2]>;
+
+// Bits of growth of a pass: log2 R, and 2 for R = 3.
+constexpr int fx_bits(int R) { return R == 16 ? 4 : R == 8 ? 3 : 2; }
+
+// Radix-R butterflies per thread of a pencil's TPP threads: j = jt + b TPP for
+// those with fx_has.
+template <class S, int R>
+constexpr int fx_bpt() { return (S::L / R + S::TPP - 1) / S::TPP; }
+template <class S, int R>
+__device__ __forceinline__ bool fx_has(int b, int jt) {
+    constexpr int NB = S::L / R;
+    return NB % S::TPP == 0 || jt + b * S::TPP < NB;
+}
+
+// K of fx_in for a pencil of bound e2 (packed: of sums of two such values).
+template <class S>
+__host__ __device__ constexpr int fx_kin(int e2, bool packed) {
+    static_assert(S::R1 == 4 || S::R1 == 8 || S::R1 == 16, "first radix");
+    return e2 + 1 + fx_bits(S::R1) + (packed ? 1 : 0);
+}
+
+// Scaling of a later pass of radix R from the largest high word h (or ~h) of
+// its inputs: times 2^l (l >= 0) and 2^-(2 + n), net 2^-d, so that the bound
+// R sqrt(2) (h + 1) 2^32 comes to at most 2^62.
+struct FxStep {
+    int l, n, d;
+};
+template <int R>
+__device__ __forceinline__ FxStep fx_step(int h) {
+    const unsigned m = (unsigned)h + 1u + (((unsigned)h + 1u) >> 1);
+    const int d = min(32 - __clz((int)m) + fx_bits(R) - 30, fx_bits(R));
+    FxStep s;
+    s.l = max(2 - d, 0);
+    s.n = max(d - 2, 0);
+    s.d = d;
+    return s;
+}
+
+// Shared words per pencil: the largest doubled high word of its input, the
+// largest high words after the first and the second pass (all zero on entry),
+// and fx_out's eb for values left in fixed point.
+constexpr int FX_WORDS = 4;
+
+// Stage the twiddle table (cos, sin of 2 pi m / L as 2^-62 (h 2^32 + l) pairs)
+// with the sign of one direction, and clear the n pencil maxima.
+template <int L, bool INV>
+__device__ __forceinline__ void fx_stage_twiddles(int4* s_tw, const int4* g_tw) {
+    for (int i = threadIdx.x; i < L; i += blockDim.x) {
+        int4 w = g_tw[i];
+        if (!INV) { w.z = -w.z; w.w = -w.w; }
+        s_tw[i] = w;
+    }
+}
+
+// Where pencil_fx takes its input from and leaves its output.
+enum FxIn { FX_IN_GLOBAL, FX_IN_TILE, FX_IN_FIXED };     // ld(e): doubles; the tile: doubles; the tile: packed fixed point
+enum FxOut { FX_OUT_GLOBAL, FX_OUT_TILE, FX_OUT_FIXED }; // st(e, value); the tile: doubles; the tile: fixed point
+
+// One later pass of radix R after NS: read, (barrier), scale, twiddle and DFT;
+// the results stay in v.  Adds the net division to eb.
+template <class S, int R, int NS, bool INV, bool SYNC>
+__device__ __forceinline__ void fx_later_pass(C<fx> (&v)[fx_bpt<S, R>()][R], const C<fx>* tile, const int4* tw, int p,
+                                              int jt, const int* hmax, int& eb, bool active) {
+    constexpr int NB = S::L / R, BPT = fx_bpt<S, R>(), STEP = S::L / (NS * R);
+    if (active) {
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                v[b][r] = fx_has<S, R>(b, jt) ? tile[S::off(jt + S::TPP * b + r * NB) + p] : mk<fx>(0, 0);
+    }
+    const FxStep st = fx_step<R>(hmax[p]);
+    if (SYNC) __syncthreads();
+    eb += st.d;
+    if (active) {
+        const fx half = (fx)(1ull << 31) << st.n;
+#pragma unroll
+        for (int b = 0; b < BPT; b++) {
+            const int k = (jt + S::TPP * b) & (NS - 1);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                v[b][r] = mk<fx>(fx_shl(v[b][r].x, st.l), fx_shl(v[b][r].y, st.l));
+                if (r > 0) v[b][r] = fx_twiddle(v[b][r], tw[(r * k) * STEP], st.n, half);
+                else v[b][r] = mk<fx>(fx_shr(v[b][r].x + (2 << st.n), st.n + 2), fx_shr(v[b][r].y + (2 << st.n), st.n + 2));
+            }
+            fx_dft<R, INV>(v[b]);
+        }
+    }
+}
+
+// Index of output r of butterfly j of a pass of radix R after NS.
+template <int R, int NS>
+__device__ __forceinline__ int fx_dest(int j) {
+    const int k = j & (NS - 1);
+    return (j - k) * R + k;
+}
+
+template <class S, int R, int NS>
+__device__ __forceinline__ void fx_write(C<fx>* tile, const C<fx> (&v)[fx_bpt<S, R>()][R], int p, int jt, unsigned zout,
+                                         int* hmax) {
+    int hi = 0, lo = 0;
+#pragma unroll
+    for (int b = 0; b < fx_bpt<S, R>(); b++) {
+        if (!fx_has<S, R>(b, jt)) continue;
+        const int d = fx_dest<R, NS>(jt + S::TPP * b);
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (!((zout >> r) & 1u)) {
+                tile[S::off(d + r * NS) + p] = v[b][r];
+                const int x = (int)(v[b][r].x >> 32), y = (int)(v[b][r].y >> 32);
+                hi = max(hi, max(x, y));
+                lo = min(lo, min(x, y));
+            }
+    }
+    if (hmax) atomicMax(hmax + p, max(hi, ~lo));
+}
+
+// The last pass's results: to st or the tile as doubles, or to the tile as they are.
+template <class S, int R, int NS, FxOut OUT, unsigned ZOUT, class St>
+__device__ __forceinline__ void fx_finish(C<double>* tile, const C<fx> (&v)[fx_bpt<S, R>()][R], int p, int jt,
+                                          FxScale sc, int eb, St st) {
+    if constexpr (OUT == FX_OUT_FIXED) {
+        fx_write<S, R, NS>(reinterpret_cast<C<fx>*>(tile), v, p, jt, ZOUT, nullptr);
+    } else {
+        constexpr int BPT = fx_bpt<S, R>();
+        C<double> o[BPT][R];
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                o[b][r] = ((ZOUT >> r) & 1u) ? mk<double>(0., 0.) : fx_out(v[b][r], eb);
+        if (sc.rare) fx_scale_all<BPT * R>(&o[0][0], fx_post(sc.rare));
+#pragma unroll
+        for (int b = 0; b < BPT; b++) {
+            if (!fx_has<S, R>(b, jt)) continue;
+            const int d = fx_dest<R, NS>(jt + S::TPP * b);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if constexpr (OUT == FX_OUT_TILE) { if (!((ZOUT >> r) & 1u)) tile[S::off(d + r * NS) + p] = o[b][r]; }
+                else st(d + r * NS, o[b][r]);
+            }
+        }
+    }
+}
+
+// Transform S::P pencils (thread: pencil p, butterflies jt + b TPP).  smax:
+// FX_WORDS arrays of P shared words, zero on entry but for the first one with
+// FX_IN_FIXED (the pencils' largest doubled high words).  The caller synchronises before, except
+// that FX_IN_GLOBAL does so itself once its loads are issued (staged twiddles
+// and cleared maxima become visible there); FX_OUT_TILE / FX_OUT_FIXED return
+// synchronised.  PRUNE as in pencil_fft_s: inputs of the removed band are
+// taken as zero, outputs in it are not computed (st gets zeros).
+// Threads with active = false only take part in the barriers.
+template <class S, bool INV, bool PRUNE, FxIn IN, FxOut OUT, class Ld, class St>
+__device__ __forceinline__ void pencil_fx(C<double>* tile, const int4* tw, unsigned* smax, Ld ld, St st, bool active = true) {
+    constexpr int L = S::L, R1 = S::R1, NB1 = L / R1, BPT1 = fx_bpt<S, R1>();
+    constexpr int NPASS = S::R3 > 1 ? 3 : S::R2 > 1 ? 2 : 1;
+    constexpr int RL = NPASS == 3 ? S::R3 : S::R2;
+    constexpr unsigned ZI = (PRUNE && INV && NPASS > 1) ? band_mask<L, R1>() : 0u;
+    constexpr unsigned ZO = (PRUNE && !INV && NPASS > 1) ? band_mask<L, RL>() : 0u;
+    const int p = active ? threadIdx.x % S::P : 0, jt = active ? threadIdx.x / S::P : 0;
+    C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
+    C<fx> v[BPT1][R1];
+    FxScale sc;
+    if constexpr (IN == FX_IN_FIXED) {
+        if (active) {
+#pragma unroll
+            for (int b = 0; b < BPT1; b++)
+#pragma unroll
+                for (int r = 0; r < R1; r++)
+                    v[b][r] = ((ZI >> r) & 1u) || !fx_has<S, R1>(b, jt) ? mk<fx>(0, 0)
+                                                                        : ft[S::off(jt + S::TPP * b + r * NB1) + p];
+        }
+        sc = fx_scale(smax[p] >> 1);
+        __syncthreads();
+    } else {
+        C<double> d[BPT1][R1];
+        if (active) {
+#pragma unroll
+            for (int b = 0; b < BPT1; b++)
+#pragma unroll
+                for (int r = 0; r < R1; r++) {
+                    const int e = jt + S::TPP * b + r * NB1;
+                    if (((ZI >> r) & 1u) || !fx_has<S, R1>(b, jt)) d[b][r] = mk<double>(0., 0.);
+                    else if constexpr (IN == FX_IN_GLOBAL) d[b][r] = ld(e);
+                    else d[b][r] = tile[S::off(e) + p];
+                }
+        }
+        if (IN == FX_IN_GLOBAL) __syncthreads();
+        if (active) {
+            unsigned h = 0;
+#pragma unroll
+            for (int b = 0; b < BPT1; b++)
+#pragma unroll
+                for (int r = 0; r < R1; r++)
+                    if (!((ZI >> r) & 1u)) h = fx_max(h, d[b][r]);
+            atomicMax(smax + p, h);
+        }
+        __syncthreads();
+        sc = fx_scale(smax[p] >> 1);
+        if (active) {
+            if (sc.rare) fx_scale_all<BPT1 * R1>(&d[0][0], fx_pre(sc.rare));
+            const int K = fx_kin<S>(sc.e2, false);
+#pragma unroll
+            for (int b = 0; b < BPT1; b++)
+#pragma unroll
+                for (int r = 0; r < R1; r++) {
+                    if ((ZI >> r) & 1u) { v[b][r] = mk<fx>(0, 0); continue; }
+                    v[b][r] = fx_in(d[b][r], K);
+                }
+        }
+    }
+    if (active) {
+#pragma unroll
+        for (int b = 0; b < BPT1; b++) fx_dft<R1, INV>(v[b]);
+    }
+    int eb = fx_kin<S>(sc.e2, IN == FX_IN_FIXED);
+    int* hm = reinterpret_cast<int*>(smax + S::P);
+    constexpr bool TO_TILE = OUT != FX_OUT_GLOBAL;
+    if constexpr (NPASS == 1) {
+        if (active) fx_finish<S, R1, 1, OUT, 0u>(tile, v, p, jt, sc, eb, st);
+    } else {
+        if (active) fx_write<S, R1, 1>(ft, v, p, jt, 0u, hm);
+        __syncthreads();
+        constexpr bool LAST2 = NPASS == 2;
+        C<fx> v2[fx_bpt<S, S::R2>()][S::R2];
+        fx_later_pass<S, S::R2, R1, INV, !LAST2 || TO_TILE>(v2, ft, tw, p, jt, hm, eb, active);
+        if constexpr (LAST2) {
+            if (active) fx_finish<S, S::R2, R1, OUT, ZO>(tile, v2, p, jt, sc, eb, st);
+        } else {
+            if (active) fx_write<S, S::R2, R1>(ft, v2, p, jt, 0u, hm + S::P);
+            __syncthreads();
+            C<fx> v3[fx_bpt<S, S::R3>()][S::R3];
+            fx_later_pass<S, S::R3, R1 * S::R2, INV, TO_TILE>(v3, ft, tw, p, jt, hm + S::P, eb, active);
+            if (active) fx_finish<S, S::R3, R1 * S::R2, OUT, ZO>(tile, v3, p, jt, sc, eb, st);
+        }
+    }
+    if (OUT == FX_OUT_FIXED && active && jt == 0) hm[2 * S::P + p] = eb;
+    if (TO_TILE) __syncthreads();
+}
+
+// --------------------------------------------------- real rows in pairs
+// Two half spectra A, B (kx < Kx) per pencil into the packed sequence
+// Z = A + iB of a c2r transform, in fixed point: each mode is loaded and
+// converted once for both of its places in Z.  get(pj, k, A, B) loads; the
+// imaginary parts at kx = 0 are dropped, as a c2r transform does.
+template <class S, int NP, int NT, class Get>
+__device__ __forceinline__ void fx_fill_packed(C<double>* tile, unsigned* smax, int Kx, Get get) {
+    constexpr int L = S::L, H = L / 2, N = H * NP, NPT = (N + NT - 1) / NT;
+    constexpr bool WARP = H % 32 == 0 && NT % 32 == 0;       // a warp's entries lie in one pencil
+    C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
+    C<double> A[NPT], B[NPT];
+#pragma unroll
+    for (int i = 0; i < NPT; i++) {
+        const int idx = threadIdx.x + i * NT, k = idx % H, pj = idx / H;
+        A[i] = B[i] = mk<double>(0., 0.);
+        if ((N % NT == 0 || idx < N) && k < Kx) get(pj, k, A[i], B[i]);
+        if (k == 0) { A[i].y = 0.; B[i].y = 0.; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NPT; i++) {
+        const int idx = threadIdx.x + i * NT, pj = idx / H;
+        unsigned h = fx_max(fx_max(0u, A[i]), B[i]);
+        if constexpr (WARP) {
+            h = __reduce_max_sync(0xffffffffu, h);
+            if ((threadIdx.x & 31) == 0 && idx < N) atomicMax(smax + pj, h);
+        } else if (N % NT == 0 || idx < N) {
+            atomicMax(smax + pj, h);
+        }
+    }
+    __syncthreads();
+    FxScale sc[NPT];
+    int rare = 0;
+#pragma unroll
+    for (int i = 0; i < NPT; i++) {
+        const int idx = threadIdx.x + i * NT;
+        sc[i] = fx_scale(N % NT == 0 || idx < N ? smax[idx / H] >> 1 : 0u);
+        rare |= sc[i].rare;
+    }
+    if (rare) {
+#pragma unroll
+        for (int i = 0; i < NPT; i++) {
+            const double pre = fx_pre(sc[i].rare);
+            A[i].x *= pre; A[i].y *= pre; B[i].x *= pre; B[i].y *= pre;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NPT; i++) {
+        const int idx = threadIdx.x + i * NT, k = idx % H, pj = idx / H;
+        if (N % NT != 0 && idx >= N) continue;
+        const int K = fx_kin<S>(sc[i].e2, true);
+        const C<fx> a = fx_in(A[i], K), b = fx_in(B[i], K);
+        ft[S::off(k) + pj] = mk<fx>(a.x - b.y, a.y + b.x);
+        ft[S::off(k == 0 ? H : L - k) + pj] = k == 0 ? mk<fx>(0, 0) : mk<fx>(a.x + b.y, b.x - a.y);
+    }
+}
+
+// The half spectra of the real rows in a tile of packed forward transforms
+// (FX_OUT_FIXED): row t is the real (t even) or imaginary part of pencil t / 2.
+// Groups of threads take the nu rows row(u) >= 0 in turn, consecutive threads
+// consecutive kx < Kx, and put(u, k, value) the spectrum times 2^sexp smul.
+template <class S, int NT, class Row, class Put>
+__device__ __forceinline__ void fx_unpack(const C<double>* tile, const unsigned* smax, int Kx, int nu, int sexp, double smul,
+                                          Row row, Put put) {
+    constexpr int G = NT % 32 == 0 ? 32 : 16;
+    static_assert(NT % G == 0, "threads come in groups");
+    const C<fx>* ft = reinterpret_cast<const C<fx>*>(tile);
+    for (int u = threadIdx.x / G; u < nu; u += NT / G) {
+        const int t = row(u);
+        if (t < 0) continue;
+        const int p = t >> 1;
+        const bool odd = t & 1;
+        const FxScale sc = fx_scale(smax[p] >> 1);
+        const int eb = (int)smax[3 * S::P + p] - 1 + sexp;
+        const auto value = [&](int k) {
+            const C<fx> z = ft[S::off(k) + p], w = ft[S::off(k == 0 ? 0 : S::L - k) + p];
+            // A = (z + conj w) / 2, B = (z - conj w) / 2i
+            const fx re = odd ? z.y + w.y : z.x + w.x, im = odd ? w.x - z.x : z.y - w.y;
+            return fx_out(mk<fx>(re, im), eb);
+        };
+        if (smul == 1.0 && !sc.rare) {
+            for (int k = threadIdx.x % G; k < Kx; k += G) put(u, k, value(k));
+        } else {
+            const double post = sc.rare ? fx_post(sc.rare) : 1.0;
+            for (int k = threadIdx.x % G; k < Kx; k += G) {
+                const C<double> o = value(k);
+                put(u, k, mk<double>((o.x * smul) * post, (o.y * smul) * post));
+            }
+        }
+    }
+}
+
+// scale = 2^sexp smul with smul = 1 for a power of two and sexp = 0 otherwise.
+inline void fx_split_scale(double scale, int& sexp, double& smul) {
+    int e;
+    const bool two = frexp(scale, &e) == 0.5;
+    sexp = two ? e - 1 : 0;
+    smul = two ? 1.0 : scale;
+}
+
+}  // namespace dd

@@ -116,6 +116,7 @@ int fft_r2c(const dd_plan* pl, int nf, const XT* const* x, void* const* k, void*
         }
         const int nrows = g.Nz * g.Ny;
         OpXr2c3<T, XT> a{nrows, g.Nx, g.Kx, s, xin, w2, TwSel<T>::x(pl)};
+        fx_split_scale(pl->inv_n, a.sexp, a.smul);
         DD_TRY((launch_pass_len<T, false, true, true>(g.Nx, a, (nrows + 1) / 2, 1, nf, st)));
         OpYFwd3<T> b{g, w2c, w1, TwSel<T>::y(pl)};
         DD_TRY((launch_pass_len<T, false, false, false>(g.Ny, b, g.Kx, g.Nz, nf, st)));
@@ -131,6 +132,7 @@ int fft_r2c(const dd_plan* pl, int nf, const XT* const* x, void* const* k, void*
         Ptrs w{}; CPtrs wc{};
         for (int f = 0; f < nf; f++) { w.p[f] = W + f * g.wcount(); wc.p[f] = w.p[f]; }
         OpXr2c3<T, XT> a{g.Ny, g.Nx, g.Kx, s, xin, w, TwSel<T>::x(pl)};
+        fx_split_scale(pl->inv_n, a.sexp, a.smul);
         DD_TRY((launch_pass_len<T, false, true, true>(g.Nx, a, (g.Ny + 1) / 2, 1, nf, st)));
         OpYFwd2<T, double> b{g, wc, ko, TwSel<T>::y(pl)};
         DD_TRY((launch_pass_len<T, false, false, true>(g.Ny, b, g.Kx, 1, nf, st)));

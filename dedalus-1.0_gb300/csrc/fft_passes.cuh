@@ -16,7 +16,7 @@
 #include <type_traits>
 #include <utility>
 
-#include "fft_engine.cuh"
+#include "fft_fixed.cuh"
 #include "geometry.cuh"
 
 namespace dd {
@@ -74,34 +74,118 @@ __device__ __forceinline__ void load_tile(const Op& op, C<T>* tile, int fld, int
     }
 }
 
-template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
-__global__ void __launch_bounds__(FFTCfg<L>::NT) k_pass(const Op op, int nfield) {
+// Index of element e of row s (rows of n elements of stride k) at kx, and of
+// element s of the e-th such row.  The register path of the FP64 passes walks e in
+// compile-time steps from one base; the staged path takes one product per entry
+// (the other way round each was 5% slower).
+template <typename T>
+__device__ __forceinline__ int64_t row_at(int s, int e, int n, int k, int kx) {
+    if constexpr (std::is_same<T, double>::value) return (int64_t)s * n * k + kx + e * k;
+    else return ((int64_t)s * n + e) * k + kx;
+}
+template <typename T>
+__device__ __forceinline__ int64_t pencil_at(int e, int s, int n, int k, int kx) {
+    if constexpr (std::is_same<T, double>::value) return (int64_t)s * k + kx + (int64_t)e * (n * k);
+    else return ((int64_t)e * n + s) * k + kx;
+}
+
+// How an Op of real rows maps to the FP64 transforms: 1 = c2r (packed half
+// spectra in), 2 = r2c (half spectra out), 0 = complex pencils.
+template <class Op> struct RealRows { static constexpr int kind = 0; };
+
+template <class Op, class = void> struct HasPut : std::false_type {};
+template <class Op>
+struct HasPut<Op, std::void_t<decltype(&Op::put)>> : std::true_type {};
+
+// Shared memory: the tile, the staged twiddles and (FP64) the pencils' scaling words.
+template <typename T, class S>
+constexpr size_t pass_smem() {
+    return S::template smem_bytes<T>() + (std::is_same<T, double>::value ? sizeof(unsigned) * FX_WORDS * S::P : 0);
+}
+
+// FP64: fixed-point transforms (fft_fixed.cuh).  Pencils that are adjacent in
+// memory go straight from global memory to the registers of the first
+// butterflies and from those of the last ones back, so that the tile is
+// written and read once per pass boundary only; contiguous pencils and real
+// rows are staged in the tile.
+template <class S, bool INV, bool LD_E, bool ST_E, bool PRUNE, class Op>
+__device__ __forceinline__ void fx_pass_body(const Op& op, C<double>* tile, const int4* tw, unsigned* smax, int fld, int s,
+                                             int f0, int npen) {
+    constexpr int L = S::L, P = S::P, PS = S::PS, NT = S::NT;
+    static_assert(S::SKD == 0, "plain tile rows");
+    const int f = f0 + threadIdx.x % P;
+    const auto ld = [&](int e) { return f < npen ? op.load(fld, s, e, f) : mk<double>(0., 0.); };
+    const auto st = [&](int e, C<double> c) { if constexpr (HasPut<Op>::value) { if (f < npen) op.put(fld, s, e, f, c); } };
+    constexpr int RR = RealRows<Op>::kind;
+    constexpr FxIn IN = RR == 1 ? FX_IN_FIXED : LD_E ? FX_IN_TILE : FX_IN_GLOBAL;
+    constexpr FxOut OUT = RR == 2 ? FX_OUT_FIXED : ST_E ? FX_OUT_TILE : FX_OUT_GLOBAL;
+    if constexpr (RR == 1) {
+        fx_fill_packed<S, P, NT>(tile, smax, op.Kx, [&](int pj, int k, C<double>& A, C<double>& B) {
+            if (f0 + pj < npen) op.load_pair(fld, k, f0 + pj, A, B);
+        });
+        __syncthreads();
+    } else if constexpr (LD_E) {
+        load_tile<double, L, P, PS, NT, true>(op, tile, fld, s, f0, npen);
+        __syncthreads();
+    }
+    pencil_fx<S, INV, PRUNE, IN, OUT>(tile, tw, smax, ld, st);
+    if constexpr (RR == 2) {
+        fx_unpack<S, NT>(tile, smax, op.Kx, 2 * P, op.sexp, op.smul,
+                         [&](int u) { return 2 * f0 + u < op.nrows ? u : -1; },
+                         [&](int u, int k, C<double> c) { op.put_row(fld, 2 * f0 + u, k, c); });
+    } else if constexpr (ST_E) {
+        const int nst = op.nstore();
+        for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
+            const int e = idx % nst, p = idx / nst;
+            if (f0 + p < npen) op.put(fld, s, e, f0 + p, tile[e * PS + p]);
+        }
+    }
+}
+
+template <typename T, class S, bool INV, bool LD_E, bool ST_E, int MB, class Op>
+__global__ void __launch_bounds__(S::NT, MB) k_pass(const Op op, int nfield) {
     extern __shared__ __align__(16) unsigned char dd_smem[];
-    constexpr int P = Pencil<L>::P, PS = Pencil<L>::PS, NT = Pencil<L>::NT;
+    constexpr int L = S::L, P = S::P, PS = S::PS, NT = S::NT;
     C<T>* tile = reinterpret_cast<C<T>*>(dd_smem);
-    C<T>* tw = tile + L * PS;
-    load_twiddles<T, L>(tw, op.tw);
     const int fld = blockIdx.x % nfield;
     const int f0 = (blockIdx.x / nfield) * P;
     const int s = blockIdx.y + 65535 * blockIdx.z;
     const int npen = op.npencil();
-    load_tile<T, L, P, PS, NT, LD_E>(op, tile, fld, s, f0, npen);
-    __syncthreads();
-    pass_fft<T, DefSched<L>, INV>(op, tile, tw);
-    const int nst = op.nstore();
-    for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
-        const int e = ST_E ? idx % nst : idx / P;
-        const int p = ST_E ? idx / nst : idx % P;
-        const int f = f0 + p;
-        if (f < npen) op.store(fld, s, e, f, tile + p, PS);
+    if constexpr (std::is_same<T, double>::value) {
+        int4* tw = reinterpret_cast<int4*>(tile + L * PS);
+        unsigned* smax = reinterpret_cast<unsigned*>(tw + L);
+        fx_stage_twiddles<L, INV>(tw, op.tw);
+        for (int i = threadIdx.x; i < FX_WORDS * P; i += NT) smax[i] = 0u;
+        if constexpr (HasKept<Op>::value) {
+            if (op.kept() == kept23(L)) {
+                fx_pass_body<S, INV, LD_E, ST_E, true>(op, tile, tw, smax, fld, s, f0, npen);
+                return;
+            }
+        }
+        fx_pass_body<S, INV, LD_E, ST_E, false>(op, tile, tw, smax, fld, s, f0, npen);
+    } else {
+        C<T>* tw = tile + L * PS;
+        load_twiddles<T, L>(tw, op.tw);
+        load_tile<T, L, P, PS, NT, LD_E>(op, tile, fld, s, f0, npen);
+        __syncthreads();
+        pass_fft<T, S, INV>(op, tile, tw);
+        const int nst = op.nstore();
+        for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
+            const int e = ST_E ? idx % nst : idx / P;
+            const int p = ST_E ? idx / nst : idx % P;
+            const int f = f0 + p;
+            if (f >= npen) continue;
+            if constexpr (HasPut<Op>::value) op.put(fld, s, e, f, tile[e * PS + p]);
+            else op.store(fld, s, e, f, tile + p, PS);
+        }
     }
 }
 
-template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
-int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
-    constexpr int P = Pencil<L>::P, NT = Pencil<L>::NT;
-    const size_t smem = Pencil<L>::template smem_bytes<T>();
-    auto kern = k_pass<T, L, INV, LD_E, ST_E, Op>;
+// MB: resident blocks per SM that the registers have to allow (0: no demand).
+template <typename T, class S, bool INV, bool LD_E, bool ST_E, int MB = 0, class Op>
+int launch_pass_sched(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st, const char* tag = "s") {
+    constexpr size_t smem = pass_smem<T, S>();
+    auto kern = k_pass<T, S, INV, LD_E, ST_E, MB, Op>;
     static std::atomic<unsigned long long> configured{0};  // per instantiation and device
     DD_TRY(ensure_smem((const void*)kern, smem, configured));
     if (npencil <= 0 || nslow <= 0 || nfield <= 0) return DD_OK;
@@ -109,53 +193,23 @@ int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t s
         set_error("pass: slow extent %d must be <= 65535 or a multiple of it", nslow);
         return DD_ERR_UNSUPPORTED;
     }
-    dim3 grid(cdiv(npencil, P) * nfield, nslow > 65535 ? 65535 : nslow, nslow > 65535 ? nslow / 65535 : 1);
-    static const std::string label = std::string(Op::name) + "_" + std::to_string(L) + PrecName<T>::s;
-    DD_KT(label.c_str(), st, kern<<<grid, NT, smem, st>>>(op, nfield));
-    DD_LAUNCH_CHECK();
-    return DD_OK;
-}
-
-// The same pass with an explicit schedule S (pencils per tile, threads, radix
-// sequence): small tiles give a small single-run grid enough blocks to fill
-// the GPU (a 128-point y pass of 43 kx pencils is 2 tiles of the default 32
-// pencils, but 11 tiles of 4).
-template <typename T, class S, bool INV, bool LD_E, bool ST_E, class Op>
-__global__ void __launch_bounds__(S::NT) k_pass_sched(const Op op, int nfield) {
-    extern __shared__ __align__(16) unsigned char dd_smem[];
-    constexpr int L = S::L, P = S::P, PS = S::PS, NT = S::NT;
-    C<T>* tile = reinterpret_cast<C<T>*>(dd_smem);
-    C<T>* tw = tile + L * PS;
-    load_twiddles<T, L>(tw, op.tw);
-    const int fld = blockIdx.x % nfield;
-    const int f0 = (blockIdx.x / nfield) * P;
-    const int s = blockIdx.y + 65535 * blockIdx.z;
-    const int npen = op.npencil();
-    load_tile<T, L, P, PS, NT, LD_E>(op, tile, fld, s, f0, npen);
-    __syncthreads();
-    pass_fft<T, S, INV>(op, tile, tw);
-    const int nst = op.nstore();
-    for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
-        const int e = ST_E ? idx % nst : idx / P;
-        const int p = ST_E ? idx / nst : idx % P;
-        const int f = f0 + p;
-        if (f < npen) op.store(fld, s, e, f, tile + p, PS);
-    }
-}
-
-template <typename T, class S, bool INV, bool LD_E, bool ST_E, class Op>
-int launch_pass_sched(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
-    const size_t smem = S::template smem_bytes<T>();
-    auto kern = k_pass_sched<T, S, INV, LD_E, ST_E, Op>;
-    static std::atomic<unsigned long long> configured{0};
-    DD_TRY(ensure_smem((const void*)kern, smem, configured));
-    if (npencil <= 0 || nslow <= 0 || nfield <= 0) return DD_OK;
-    DD_CHECK_ARG(nslow <= 65535, "pass: slow extent %d must be <= 65535", nslow);
-    dim3 grid(cdiv(npencil, S::P) * nfield, nslow, 1);
-    static const std::string label = std::string(Op::name) + "_" + std::to_string(S::L) + "s" + PrecName<T>::s;
+    dim3 grid(cdiv(npencil, S::P) * nfield, nslow > 65535 ? 65535 : nslow, nslow > 65535 ? nslow / 65535 : 1);
+    static const std::string label = std::string(Op::name) + "_" + std::to_string(S::L) + tag + PrecName<T>::s;
     DD_KT(label.c_str(), st, kern<<<grid, S::NT, smem, st>>>(op, nfield));
     DD_LAUNCH_CHECK();
     return DD_OK;
+}
+
+// The pass with the default schedule of its length.  An explicit one (pencils
+// per tile, threads, radix sequence) gives a small single-run grid enough
+// blocks to fill the GPU: a 128-point y pass of 43 kx pencils is 2 tiles of the
+// default 32 pencils, but 11 tiles of 4.
+template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
+int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
+    if constexpr (std::is_same<T, double>::value)
+        return launch_pass_sched<T, FxS<L, INV>, INV, LD_E, ST_E, FxCfg<L>::MB>(op, npencil, nslow, nfield, st, "");
+    else
+        return launch_pass_sched<T, DefSched<L>, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st, "");
 }
 
 // Small-tile schedules (4 pencils, 16 threads each) for single-run 2D grids.
@@ -187,6 +241,13 @@ template <> struct YVariant<256, 1> { using S = Sched<256, 4, 64, 16, 16, 1>; };
 template <> struct YVariant<256, 2> { using S = Sched<256, 8, 128, 16, 16, 1>; };
 template <> struct YVariant<512, 1> { using S = Sched<512, 2, 64, 8, 8, 8>; };
 template <> struct YVariant<512, 2> { using S = Sched<512, 4, 128, 8, 8, 8>; };
+template <typename T, int L, int V, bool INV>
+struct YSchedOf { using S = typename YVariant<L, V>::S; };
+template <int L, int V, bool INV>
+struct YSchedOf<double, L, V, INV> {
+    static constexpr int P = L <= 128 ? 4 * V : 2 * V;
+    using S = FxS<L, INV, P>;
+};
 
 // Launch a pass with tile variant v (1 or 2) of length L; returns 1 (not
 // launched) when no variant exists.
@@ -194,7 +255,7 @@ template <typename T, bool INV, bool LD_E, bool ST_E, class Op>
 int launch_pass_variant(int L, int v, const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
 #define DD_YV(N, VV) \
     if (L == N && v == VV) \
-        return launch_pass_sched<T, typename YVariant<N, VV>::S, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st);
+        return launch_pass_sched<T, typename YSchedOf<T, N, VV, INV>::S, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st);
     DD_YV(64, 1) DD_YV(64, 2) DD_YV(128, 1) DD_YV(128, 2) DD_YV(256, 1) DD_YV(256, 2) DD_YV(512, 1) DD_YV(512, 2)
 #undef DD_YV
     return 1;
@@ -208,18 +269,18 @@ struct OpZInv3 {
     static constexpr const char* name = "z_inv";
     static constexpr int lmin = 8, lmax = 512;
     using KV = typename Vec2<KT>::type;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw;
+    Geo3 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.Mz; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Nz; }
     __device__ C<T> load(int fld, int kyc, int e, int kx) const {
         if (!kept_full(e, g.Nz, g.Mz)) return zero<T>();
         const int ky = compact_to_full(kyc, g.Ny, g.Ky);
-        const KV v = ((const KV*)in.p[fld])[((int64_t)ky * g.Nz + e) * g.Nh + kx];
+        const KV v = ((const KV*)in.p[fld])[row_at<T>(ky, e, g.Nz, g.Nh, kx)];
         return mk<T>((T)v.x, (T)v.y);
     }
-    __device__ void store(int fld, int kyc, int e, int kx, const C<T>* col, int PS) const {
-        stc<T>((V*)out.p[fld] + ((int64_t)kyc * g.Nz + e) * g.Kx + kx, col[e * PS]);
+    __device__ void put(int fld, int kyc, int e, int kx, const C<T>& c) const {
+        stc<T>((V*)out.p[fld] + row_at<T>(kyc, e, g.Nz, g.Kx, kx), c);
     }
 };
 
@@ -229,17 +290,17 @@ struct OpYInv3 {
     using V = typename Vec2<T>::type;
     static constexpr const char* name = "y_inv";
     static constexpr int lmin = 8, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw;
+    Geo3 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.My; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<T> load(int fld, int z, int e, int kx) const {
         if (!kept_full(e, g.Ny, g.My)) return zero<T>();
         const int kyc = full_to_compact(e, g.Ny, g.Ky);
-        return ldc<T>((const V*)in.p[fld] + ((int64_t)kyc * g.Nz + z) * g.Kx + kx);
+        return ldc<T>((const V*)in.p[fld] + pencil_at<T>(kyc, z, g.Nz, g.Kx, kx));
     }
-    __device__ void store(int fld, int z, int e, int kx, const C<T>* col, int PS) const {
-        stc<T>((V*)out.p[fld] + ((int64_t)z * g.Ny + e) * g.Kx + kx, col[e * PS]);
+    __device__ void put(int fld, int z, int e, int kx, const C<T>& c) const {
+        stc<T>((V*)out.p[fld] + row_at<T>(z, e, g.Ny, g.Kx, kx), c);
     }
 };
 
@@ -277,7 +338,7 @@ struct OpXc2r3 {
     using V = typename Vec2<T>::type;
     static constexpr const char* name = "x_c2r";
     static constexpr int lmin = 8, lmax = 512;
-    int nrows, Nx, Kx; CPtrs in; Ptrs out; const V* tw;
+    int nrows, Nx, Kx; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return Kx - 1; }
     __device__ int npencil() const { return (nrows + 1) / 2; }
     __device__ int nstore() const { return Nx; }
@@ -288,9 +349,14 @@ struct OpXc2r3 {
         if (rb == ra) z.y = T(0);
         return z;
     }
-    __device__ void store(int fld, int, int e, int f, const C<T>* col, int PS) const {
+    // the half spectra of pencil f's two rows at kx = k
+    __device__ void load_pair(int fld, int k, int f, C<T>& A, C<T>& B) const {
+        const V* W = (const V*)in.p[fld] + (int64_t)(2 * f) * Kx + k;
+        A = ldc<T>(W);
+        if (2 * f + 1 < nrows) B = ldc<T>(W + Kx);
+    }
+    __device__ void put(int fld, int, int e, int f, const C<T>& v) const {
         XT* x = (XT*)out.p[fld];
-        const C<T> v = col[e * PS];
         x[(int64_t)(2 * f) * Nx + e] = (XT)v.x;
         if (2 * f + 1 < nrows) x[(int64_t)(2 * f + 1) * Nx + e] = (XT)v.y;
     }
@@ -303,7 +369,8 @@ struct OpXr2c3 {
     using V = typename Vec2<T>::type;
     static constexpr const char* name = "x_r2c";
     static constexpr int lmin = 8, lmax = 512;
-    int nrows, Nx, Kx; T s; CPtrs in; Ptrs out; const V* tw;
+    int nrows, Nx, Kx; T s; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
+    int sexp = 0; double smul = 1.0;       // s = 2^sexp smul (fx_split_scale; FP64 only)
     __device__ int kept() const { return Kx - 1; }
     __device__ int npencil() const { return (nrows + 1) / 2; }
     __device__ int nstore() const { return Kx; }
@@ -320,7 +387,10 @@ struct OpXr2c3 {
         stc<T>(W + (int64_t)(2 * f) * Kx + k, A);
         if (2 * f + 1 < nrows) stc<T>(W + (int64_t)(2 * f + 1) * Kx + k, B);
     }
+    __device__ void put_row(int fld, int row, int k, C<T> c) const { stc<T>((V*)out.p[fld] + (int64_t)row * Kx + k, c); }
 };
+template <typename XT> struct RealRows<OpXc2r3<double, XT>> { static constexpr int kind = 1; };
+template <typename XT> struct RealRows<OpXr2c3<double, XT>> { static constexpr int kind = 2; };
 
 // Forward along y: W2[z][y][kxc] -> W1[kyc][z][kxc] (kept ky only).
 template <typename T>
@@ -328,17 +398,17 @@ struct OpYFwd3 {
     using V = typename Vec2<T>::type;
     static constexpr const char* name = "y_fwd";
     static constexpr int lmin = 8, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw;
+    Geo3 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.My; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<T> load(int fld, int z, int e, int kx) const {
-        return ldc<T>((const V*)in.p[fld] + ((int64_t)z * g.Ny + e) * g.Kx + kx);
+        return ldc<T>((const V*)in.p[fld] + row_at<T>(z, e, g.Ny, g.Kx, kx));
     }
-    __device__ void store(int fld, int z, int e, int kx, const C<T>* col, int PS) const {
+    __device__ void put(int fld, int z, int e, int kx, const C<T>& c) const {
         if (!kept_full(e, g.Ny, g.My)) return;
         const int kyc = full_to_compact(e, g.Ny, g.Ky);
-        stc<T>((V*)out.p[fld] + ((int64_t)kyc * g.Nz + z) * g.Kx + kx, col[e * PS]);
+        stc<T>((V*)out.p[fld] + pencil_at<T>(kyc, z, g.Nz, g.Kx, kx), c);
     }
 };
 
@@ -350,19 +420,19 @@ struct OpZFwd3 {
     static constexpr const char* name = "z_fwd";
     static constexpr int lmin = 8, lmax = 512;
     using KV = typename Vec2<KT>::type;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw;
+    Geo3 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.Mz; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Nz; }
     __device__ C<T> load(int fld, int kyc, int e, int kx) const {
-        return ldc<T>((const V*)in.p[fld] + ((int64_t)kyc * g.Nz + e) * g.Kx + kx);
+        return ldc<T>((const V*)in.p[fld] + row_at<T>(kyc, e, g.Nz, g.Kx, kx));
     }
-    __device__ void store(int fld, int kyc, int e, int kx, const C<T>* col, int PS) const {
+    __device__ void put(int fld, int kyc, int e, int kx, const C<T>& c) const {
         const int ky = compact_to_full(kyc, g.Ny, g.Ky);
         KV v;
-        if (kept_full(e, g.Nz, g.Mz)) { const C<T> c = col[e * PS]; v.x = (KT)c.x; v.y = (KT)c.y; }
+        if (kept_full(e, g.Nz, g.Mz)) {  v.x = (KT)c.x; v.y = (KT)c.y; }
         else { v.x = KT(0); v.y = KT(0); }
-        ((KV*)out.p[fld])[((int64_t)ky * g.Nz + e) * g.Nh + kx] = v;
+        ((KV*)out.p[fld])[row_at<T>(ky, e, g.Nz, g.Nh, kx)] = v;
     }
 };
 
@@ -374,7 +444,7 @@ struct OpYInv2 {
     static constexpr const char* name = "y_inv2d";
     static constexpr int lmin = 8, lmax = 512;
     using KV = typename Vec2<KT>::type;
-    Geo2 g; CPtrs in; Ptrs out; const V* tw;
+    Geo2 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.My; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
@@ -383,8 +453,8 @@ struct OpYInv2 {
         const KV v = ((const KV*)in.p[fld])[(int64_t)kx * g.Ny + e];
         return mk<T>((T)v.x, (T)v.y);
     }
-    __device__ void store(int fld, int, int e, int kx, const C<T>* col, int PS) const {
-        stc<T>((V*)out.p[fld] + (int64_t)e * g.Kx + kx, col[e * PS]);
+    __device__ void put(int fld, int, int e, int kx, const C<T>& c) const {
+        stc<T>((V*)out.p[fld] + row_at<T>(0, e, 0, g.Kx, kx), c);
     }
 };
 
@@ -395,16 +465,16 @@ struct OpYFwd2 {
     static constexpr const char* name = "y_fwd2d";
     static constexpr int lmin = 8, lmax = 512;
     using KV = typename Vec2<KT>::type;
-    Geo2 g; CPtrs in; Ptrs out; const V* tw;
+    Geo2 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.My; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<T> load(int fld, int, int e, int kx) const {
-        return ldc<T>((const V*)in.p[fld] + (int64_t)e * g.Kx + kx);
+        return ldc<T>((const V*)in.p[fld] + row_at<T>(0, e, 0, g.Kx, kx));
     }
-    __device__ void store(int fld, int, int e, int kx, const C<T>* col, int PS) const {
+    __device__ void put(int fld, int, int e, int kx, const C<T>& c) const {
         KV v;
-        if (kept_full(e, g.Ny, g.My)) { const C<T> c = col[e * PS]; v.x = (KT)c.x; v.y = (KT)c.y; }
+        if (kept_full(e, g.Ny, g.My)) {  v.x = (KT)c.x; v.y = (KT)c.y; }
         else { v.x = KT(0); v.y = KT(0); }
         ((KV*)out.p[fld])[(int64_t)kx * g.Ny + e] = v;
     }

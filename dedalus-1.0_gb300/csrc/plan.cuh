@@ -17,9 +17,10 @@ struct dd_plan {
     float* kxf;
     float* kyf;
     float* kzf;
-    // twiddle tables W_L^m, m < L, per axis length (device): fp64 and fp32 as
-    // (g, t) with W = g (1 + i t) for the FMA butterflies, double-float as (cos, sin)
-    double2* tw64_x; double2* tw64_y; double2* tw64_z;
+    // twiddle tables W_L^m, m < L, per axis length (device): fp64 as (cos, sin)
+    // in 62-bit fixed point, fp32 as (g, t) with W = g (1 + i t) for the FMA
+    // butterflies, double-float as (cos, sin)
+    int4* tw64_x; int4* tw64_y; int4* tw64_z;
     float2* tw32_x;  float2* tw32_y;  float2* tw32_z;
     float4* twdf_x;  float4* twdf_y;  float4* twdf_z;   // double-float (hi, lo) pairs
     // rounded-down 1/N_total used by the forward transform
@@ -32,9 +33,9 @@ namespace dd {
 
 template <typename T> struct TwSel;
 template <> struct TwSel<double> {
-    static const double2* x(const dd_plan* p) { return p->tw64_x; }
-    static const double2* y(const dd_plan* p) { return p->tw64_y; }
-    static const double2* z(const dd_plan* p) { return p->tw64_z; }
+    static const int4* x(const dd_plan* p) { return p->tw64_x; }
+    static const int4* y(const dd_plan* p) { return p->tw64_y; }
+    static const int4* z(const dd_plan* p) { return p->tw64_z; }
 };
 template <> struct TwSel<float> {
     static const float2* x(const dd_plan* p) { return p->tw32_x; }

@@ -50,7 +50,7 @@ struct OpYInvPhys2 {
     static constexpr const char* name = PHYS == PHYS_HYDRO ? "y_inv_hydro2d" : PHYS == PHYS_BOUSS ? "y_inv_bouss2d"
                                         : PHYS == PHYS_HYDRO_DIV ? "y_inv_hydro2d_div" : "y_inv_bouss2d_div";
     static constexpr int lmin = 32, lmax = 512;
-    Geo2 g; CPtrs st; int64_t st_rs; Ptrs out; int64_t w_rs; const V* tw;
+    Geo2 g; CPtrs st; int64_t st_rs; Ptrs out; int64_t w_rs; const typename TwVec<T>::type* tw;
     const double* kx; const double* ky;
     __device__ int kept() const { return g.My; }
     __device__ int npencil() const { return g.Kx; }
@@ -77,8 +77,8 @@ struct OpYInvPhys2 {
         else r = ideriv2(get(2, run, ix, e), ky[e]);
         return mk<T>((T)r.x, (T)r.y);
     }
-    __device__ void store(int fld, int run, int e, int ix, const C<T>* col, int PS) const {
-        stc<T>((V*)out.p[fld] + run * w_rs + (int64_t)e * g.Kx + ix, col[e * PS]);
+    __device__ void put(int fld, int run, int e, int ix, const C<T>& c) const {
+        stc<T>((V*)out.p[fld] + run * w_rs + (int64_t)e * g.Kx + ix, c);
     }
 };
 
@@ -132,16 +132,15 @@ struct OpYFwdCompact2 {
     using V = typename Vec2<T>::type;
     static constexpr const char* name = "y_fwd_compact2d";
     static constexpr int lmin = 32, lmax = 512;
-    Geo2 g; CPtrs in; int64_t w_rs; Ptrs out; int64_t nc_rs; const V* tw;
+    Geo2 g; CPtrs in; int64_t w_rs; Ptrs out; int64_t nc_rs; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.My; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<T> load(int fld, int run, int e, int ix) const {
         return ldc<T>((const V*)in.p[fld] + run * w_rs + (int64_t)e * g.Kx + ix);
     }
-    __device__ void store(int fld, int run, int e, int ix, const C<T>* col, int PS) const {
+    __device__ void put(int fld, int run, int e, int ix, const C<T>& c) const {
         if (!kept_full(e, g.Ny, g.My)) return;
-        const C<T> c = col[e * PS];
         const int64_t o = run * nc_rs + (int64_t)ix * g.Ky + full_to_compact(e, g.Ny, g.Ky);
         if constexpr (std::is_same<ST, float>::value) ((float2*)out.p[fld])[o] = make_float2((float)c.x, (float)c.y);
         else ((double2*)out.p[fld])[o] = make_double2((double)c.x, (double)c.y);

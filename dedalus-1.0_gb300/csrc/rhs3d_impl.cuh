@@ -57,7 +57,7 @@ struct OpZInvCurl3 {
     using V = typename Vec2<T>::type;
     static constexpr const char* name = NG == 1 ? "z_inv_curl" : (CURL ? "z_inv_curl_mhd" : "z_inv_mhd");
     static constexpr int lmin = 16, lmax = 512;
-    Geo3 g; CPtrs u; Ptrs out; const V* tw;
+    Geo3 g; CPtrs u; Ptrs out; const typename TwVec<T>::type* tw;
     const double* kx; const double* ky; const double* kz;
     __device__ int kept() const { return g.Mz; }
     __device__ int npencil() const { return g.Kx; }
@@ -65,10 +65,10 @@ struct OpZInvCurl3 {
     __device__ double2 get(int c, int kyc, int ky_i, int e, int ix) const {
         if (COMPACT) {
             using SV = typename Vec2<ST>::type;
-            const SV v = ((const SV*)u.p[c])[((int64_t)kyc * g.Kz + full_to_compact(e, g.Nz, g.Kz)) * g.Kx + ix];
+            const SV v = ((const SV*)u.p[c])[row_at<T>(kyc, full_to_compact(e, g.Nz, g.Kz), g.Kz, g.Kx, ix)];
             return make_double2((double)v.x, (double)v.y);
         }
-        return ((const double2*)u.p[c])[((int64_t)ky_i * g.Nz + e) * g.Nh + ix];
+        return ((const double2*)u.p[c])[row_at<T>(ky_i, e, g.Nz, g.Nh, ix)];
     }
     __device__ C<T> load(int fld, int kyc, int e, int ix) const {
         if (!kept_full(e, g.Nz, g.Mz)) return zero<T>();
@@ -91,8 +91,8 @@ struct OpZInvCurl3 {
         }
         return mk<T>((T)r.x, (T)r.y);
     }
-    __device__ void store(int fld, int kyc, int e, int ix, const C<T>* col, int PS) const {
-        stc<T>((V*)out.p[fld] + ((int64_t)kyc * g.Nz + e) * g.Kx + ix, col[e * PS]);
+    __device__ void put(int fld, int kyc, int e, int ix, const C<T>& c) const {
+        stc<T>((V*)out.p[fld] + row_at<T>(kyc, e, g.Nz, g.Kx, ix), c);
     }
 };
 
@@ -180,18 +180,17 @@ struct OpZFwdCompact3 {
     using SV = typename Vec2<ST>::type;
     static constexpr const char* name = "z_fwd_compact";
     static constexpr int lmin = 16, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw;
+    Geo3 g; CPtrs in; Ptrs out; const typename TwVec<T>::type* tw;
     __device__ int kept() const { return g.Mz; }
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Nz; }
     __device__ C<T> load(int fld, int kyc, int e, int kx) const {
-        return ldc<T>((const V*)in.p[fld] + ((int64_t)kyc * g.Nz + e) * g.Kx + kx);
+        return ldc<T>((const V*)in.p[fld] + row_at<T>(kyc, e, g.Nz, g.Kx, kx));
     }
-    __device__ void store(int fld, int kyc, int e, int kx, const C<T>* col, int PS) const {
+    __device__ void put(int fld, int kyc, int e, int kx, const C<T>& c) const {
         if (!kept_full(e, g.Nz, g.Mz)) return;
-        const C<T> c = col[e * PS];
         SV v; v.x = (ST)c.x; v.y = (ST)c.y;
-        ((SV*)out.p[fld])[((int64_t)kyc * g.Kz + full_to_compact(e, g.Nz, g.Kz)) * g.Kx + kx] = v;
+        ((SV*)out.p[fld])[row_at<T>(kyc, full_to_compact(e, g.Nz, g.Kz), g.Kz, g.Kx, kx)] = v;
     }
 };
 

@@ -38,15 +38,15 @@ struct OpYFwd3S {
     using V = double2;
     static constexpr const char* name = "y_fwd_shear";
     static constexpr int lmin = 8, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw; const double* pr; double t;
+    Geo3 g; CPtrs in; Ptrs out; const int4* tw; const double* pr; double t;
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<double> load(int fld, int z, int e, int kx) const {
         const C<double> v = ldc<double>((const V*)in.p[fld] + ((int64_t)z * g.Ny + e) * g.Kx + kx);
         return shear_rot(v, pr[(int64_t)e * g.Nh + kx] * t, false);
     }
-    __device__ void store(int fld, int z, int e, int kx, const C<double>* col, int PS) const {
-        stc<double>((V*)out.p[fld] + ((int64_t)e * g.Nz + z) * g.Kx + kx, col[e * PS]);
+    __device__ void put(int fld, int z, int e, int kx, const C<double>& c) const {
+        stc<double>((V*)out.p[fld] + ((int64_t)e * g.Nz + z) * g.Kx + kx, c);
     }
 };
 
@@ -55,16 +55,16 @@ struct OpZFwd3S {
     using V = double2;
     static constexpr const char* name = "z_fwd_shear";
     static constexpr int lmin = 8, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw; const double* kys; double cut;
+    Geo3 g; CPtrs in; Ptrs out; const int4* tw; const double* kys; double cut;
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Nz; }
     __device__ C<double> load(int fld, int ky, int e, int kx) const {
         return ldc<double>((const V*)in.p[fld] + ((int64_t)ky * g.Nz + e) * g.Kx + kx);
     }
-    __device__ void store(int fld, int ky, int e, int kx, const C<double>* col, int PS) const {
+    __device__ void put(int fld, int ky, int e, int kx, const C<double>& c) const {
         const bool keep = kept_full(e, g.Nz, g.Mz) && !shear_cut(kys[(int64_t)ky * g.Nh + kx], cut);
-        const C<double> c = keep ? col[e * PS] : mk<double>(0., 0.);
-        ((V*)out.p[fld])[((int64_t)ky * g.Nz + e) * g.Nh + kx] = make_double2(c.x, c.y);
+        const C<double> o = keep ? c : mk<double>(0., 0.);
+        ((V*)out.p[fld])[((int64_t)ky * g.Nz + e) * g.Nh + kx] = make_double2(o.x, o.y);
     }
 };
 
@@ -73,15 +73,15 @@ struct OpZInv3S {
     using V = double2;
     static constexpr const char* name = "z_inv_shear";
     static constexpr int lmin = 8, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw; const double* kys; double cut;
+    Geo3 g; CPtrs in; Ptrs out; const int4* tw; const double* kys; double cut;
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Nz; }
     __device__ C<double> load(int fld, int ky, int e, int kx) const {
         if (!kept_full(e, g.Nz, g.Mz) || shear_cut(kys[(int64_t)ky * g.Nh + kx], cut)) return mk<double>(0., 0.);
         return ldc<double>((const V*)in.p[fld] + ((int64_t)ky * g.Nz + e) * g.Nh + kx);
     }
-    __device__ void store(int fld, int ky, int e, int kx, const C<double>* col, int PS) const {
-        stc<double>((V*)out.p[fld] + ((int64_t)ky * g.Nz + e) * g.Kx + kx, col[e * PS]);
+    __device__ void put(int fld, int ky, int e, int kx, const C<double>& c) const {
+        stc<double>((V*)out.p[fld] + ((int64_t)ky * g.Nz + e) * g.Kx + kx, c);
     }
 };
 
@@ -90,15 +90,15 @@ struct OpYInv3S {
     using V = double2;
     static constexpr const char* name = "y_inv_shear";
     static constexpr int lmin = 8, lmax = 512;
-    Geo3 g; CPtrs in; Ptrs out; const V* tw; const double* pr; double t;
+    Geo3 g; CPtrs in; Ptrs out; const int4* tw; const double* pr; double t;
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<double> load(int fld, int z, int e, int kx) const {
         return ldc<double>((const V*)in.p[fld] + ((int64_t)e * g.Nz + z) * g.Kx + kx);
     }
-    __device__ void store(int fld, int z, int e, int kx, const C<double>* col, int PS) const {
+    __device__ void put(int fld, int z, int e, int kx, const C<double>& c) const {
         stc<double>((V*)out.p[fld] + ((int64_t)z * g.Ny + e) * g.Kx + kx,
-                    shear_rot(col[e * PS], pr[(int64_t)e * g.Nh + kx] * t, true));
+                    shear_rot(c, pr[(int64_t)e * g.Nh + kx] * t, true));
     }
 };
 
@@ -108,17 +108,17 @@ struct OpYFwd2S {
     using V = double2;
     static constexpr const char* name = "y_fwd2d_shear";
     static constexpr int lmin = 8, lmax = 512;
-    Geo2 g; CPtrs in; Ptrs out; const V* tw; const double* pr; double t; const double* kys; double cut;
+    Geo2 g; CPtrs in; Ptrs out; const int4* tw; const double* pr; double t; const double* kys; double cut;
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<double> load(int fld, int, int e, int kx) const {
         const C<double> v = ldc<double>((const V*)in.p[fld] + (int64_t)e * g.Kx + kx);
         return shear_rot(v, pr[(int64_t)e * g.Nh + kx] * t, false);
     }
-    __device__ void store(int fld, int, int e, int kx, const C<double>* col, int PS) const {
+    __device__ void put(int fld, int, int e, int kx, const C<double>& c) const {
         const bool keep = !shear_cut(kys[(int64_t)kx * g.Ny + e], cut);
-        const C<double> c = keep ? col[e * PS] : mk<double>(0., 0.);
-        ((V*)out.p[fld])[(int64_t)kx * g.Ny + e] = make_double2(c.x, c.y);
+        const C<double> o = keep ? c : mk<double>(0., 0.);
+        ((V*)out.p[fld])[(int64_t)kx * g.Ny + e] = make_double2(o.x, o.y);
     }
 };
 
@@ -127,16 +127,16 @@ struct OpYInv2S {
     using V = double2;
     static constexpr const char* name = "y_inv2d_shear";
     static constexpr int lmin = 8, lmax = 512;
-    Geo2 g; CPtrs in; Ptrs out; const V* tw; const double* pr; double t; const double* kys; double cut;
+    Geo2 g; CPtrs in; Ptrs out; const int4* tw; const double* pr; double t; const double* kys; double cut;
     __device__ int npencil() const { return g.Kx; }
     __device__ int nstore() const { return g.Ny; }
     __device__ C<double> load(int fld, int, int e, int kx) const {
         if (shear_cut(kys[(int64_t)kx * g.Ny + e], cut)) return mk<double>(0., 0.);
         return ldc<double>((const V*)in.p[fld] + (int64_t)kx * g.Ny + e);
     }
-    __device__ void store(int fld, int, int e, int kx, const C<double>* col, int PS) const {
+    __device__ void put(int fld, int, int e, int kx, const C<double>& c) const {
         stc<double>((V*)out.p[fld] + (int64_t)e * g.Kx + kx,
-                    shear_rot(col[e * PS], pr[(int64_t)e * g.Nh + kx] * t, true));
+                    shear_rot(c, pr[(int64_t)e * g.Nh + kx] * t, true));
     }
 };
 
@@ -269,6 +269,7 @@ int dd_shear_r2c(const dd_plan* p, int nfield, const double* const* x, void* con
         }
         const int nrows = g.Nz * g.Ny;
         OpXr2c3<double, double> a{nrows, g.Nx, g.Kx, s, xin, w2, TwSel<double>::x(p)};
+        fx_split_scale(p->inv_n, a.sexp, a.smul);
         DD_TRY((launch_pass_len<double, false, true, true>(g.Nx, a, (nrows + 1) / 2, 1, nfield, st)));
         OpYFwd3S b{g, w2c, ws, TwSel<double>::y(p), pr, t};
         DD_TRY((launch_pass_len<double, false, false, false>(g.Ny, b, g.Kx, g.Nz, nfield, st)));
@@ -286,6 +287,7 @@ int dd_shear_r2c(const dd_plan* p, int nfield, const double* const* x, void* con
         CPtrs wc{};
         for (int f = 0; f < nfield; f++) { w.p[f] = W + f * g.wcount(); wc.p[f] = w.p[f]; }
         OpXr2c3<double, double> a{g.Ny, g.Nx, g.Kx, s, xin, w, TwSel<double>::x(p)};
+        fx_split_scale(p->inv_n, a.sexp, a.smul);
         DD_TRY((launch_pass_len<double, false, true, true>(g.Nx, a, (g.Ny + 1) / 2, 1, nfield, st)));
         OpYFwd2S b{g, wc, ko, TwSel<double>::y(p), pr, t, kys, cut};
         DD_TRY((launch_pass_len<double, false, false, true>(g.Ny, b, g.Kx, 1, nfield, st)));
