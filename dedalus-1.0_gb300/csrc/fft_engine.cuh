@@ -33,6 +33,8 @@
 //
 // Forward transforms use exp(-i...), inverse exp(+i...); neither is scaled.
 #pragma once
+#include <type_traits>
+
 #include "dd_common.cuh"
 #include "df64.cuh"
 
@@ -409,16 +411,6 @@ struct Sched {
 template <int L>
 using DefSched = Sched<L, FFTCfg<L>::P, FFTCfg<L>::NT, FFTCfg<L>::R1, FFTCfg<L>::R2, FFTCfg<L>::R3>;
 
-template <int L>
-struct Pencil {
-    static constexpr int P = FFTCfg<L>::P;
-    static constexpr int NT = FFTCfg<L>::NT;
-    static constexpr int PS = DefSched<L>::PS;
-    static constexpr int TPP = NT / P;
-    template <typename T>
-    static constexpr size_t smem_bytes() { return DefSched<L>::template smem_bytes<T>(); }
-};
-
 // One Stockham pass of radix R with current sub-transform length NS.  tw is
 // the staged twiddle table: (g, t) pairs for FP32, (cos, sin) for double-float.
 template <typename T, class S, int R, int NS, bool INV, unsigned ZIN = 0u, unsigned ZOUT = 0u>
@@ -505,9 +497,87 @@ __device__ __forceinline__ void pencil_fft_s(C<T>* tile, const C<T>* tw, bool ac
     }
 }
 
-template <typename T, int L, bool INV>
-__device__ __forceinline__ void pencil_fft(C<T>* tile, const C<T>* tw) {
-    pencil_fft_s<T, DefSched<L>, INV>(tile, tw);
+// The same transform with the first pass's inputs from ld(e) (DIN) and the last
+// pass's outputs to st(e, value) (DOUT) instead of the tile: the tile is then
+// written and read once per pass boundary only.  With DIN the first barrier
+// comes after the first pass (the staged twiddles are not read before it).
+// st gets zeros in the band that PRUNE removes.
+template <typename T, class S, bool INV, bool PRUNE, bool DIN, bool DOUT, class Ld, class St>
+__device__ __forceinline__ void pencil_fft_io(C<T>* tile, const C<T>* tw, Ld ld, St st) {
+    constexpr int L = S::L, TPP = S::TPP;
+    constexpr int NPASS = S::R3 > 1 ? 3 : S::R2 > 1 ? 2 : 1;
+    constexpr int RL = NPASS == 3 ? S::R3 : NPASS == 2 ? S::R2 : S::R1, NSL = L / RL;
+    constexpr bool PR = PRUNE && IsLF<T>::value && NPASS > 1;
+    constexpr unsigned ZI = (PR && INV) ? band_mask<L, S::R1>() : 0u;
+    constexpr unsigned ZO = (PR && !INV) ? band_mask<L, RL>() : 0u;
+    static_assert(S::SKD == 0, "plain tile rows");
+    const int p = threadIdx.x % S::P, jt = threadIdx.x / S::P;
+    // butterflies of one pass, in registers
+    const auto bfly = [&](auto& v, auto radix, auto ns, auto zi, auto zo, int k) {
+        constexpr int R = decltype(radix)::value, NS = decltype(ns)::value;
+        constexpr unsigned zin = decltype(zi)::value, zout = decltype(zo)::value;
+        if constexpr (IsLF<T>::value) {
+            bfly_lf<R, NS, L, INV, zin, zout>(v, tw, k);
+        } else {
+            if constexpr (NS > 1) {
+#pragma unroll
+                for (int r = 1; r < R; r++) {
+                    const C<T> w = tw[(r * k) * (L / (NS * R))];
+                    v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
+                }
+            }
+            dft<R, INV>(v);
+        }
+    };
+    {
+        constexpr int R = S::R1, NB = L / R, BPT = NB / TPP;
+        C<T> v[BPT][R];
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int e = jt + TPP * b + r * NB;
+                if ((ZI >> r) & 1u) v[b][r] = zero<T>();
+                else if constexpr (DIN) v[b][r] = ld(e);
+                else v[b][r] = tile[S::off(e) + p];
+            }
+        if (!DIN && (NPASS > 1 || !DOUT)) __syncthreads();
+#pragma unroll
+        for (int b = 0; b < BPT; b++) {
+            const int j = jt + TPP * b;
+            bfly(v[b], std::integral_constant<int, R>{}, std::integral_constant<int, 1>{},
+                 std::integral_constant<unsigned, ZI>{}, std::integral_constant<unsigned, 0u>{}, 0);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if constexpr (NPASS == 1 && DOUT) st(j * R + r, v[b][r]);
+                else tile[S::off(j * R + r) + p] = v[b][r];
+            }
+        }
+        if (NPASS > 1 || !DOUT) __syncthreads();
+    }
+    if constexpr (NPASS == 3) stockham_pass<T, S, S::R2, S::R1, INV>(tile, tw, p, jt);
+    if constexpr (NPASS > 1) {
+        constexpr int R = RL, NB = L / R, BPT = NB / TPP;
+        C<T> v[BPT][R];
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R; r++) v[b][r] = tile[S::off(jt + TPP * b + r * NB) + p];
+        if (!DOUT) __syncthreads();
+#pragma unroll
+        for (int b = 0; b < BPT; b++) {
+            const int j = jt + TPP * b, k = j & (NSL - 1), d = (j - k) * R + k;
+            bfly(v[b], std::integral_constant<int, R>{}, std::integral_constant<int, NSL>{},
+                 std::integral_constant<unsigned, 0u>{}, std::integral_constant<unsigned, ZO>{}, k);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const bool dropped = (ZO >> r) & 1u;
+                if constexpr (DOUT) st(d + r * NSL, dropped ? zero<T>() : v[b][r]);
+                else if (!dropped) tile[S::off(d + r * NSL) + p] = v[b][r];
+            }
+        }
+        if (!DOUT) __syncthreads();
+    }
 }
 
 // Stage the length-L twiddle table (global, L entries) into shared memory.

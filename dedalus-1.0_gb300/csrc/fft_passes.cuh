@@ -10,8 +10,13 @@
 // working on the same tile for different fields run together and re-reads of
 // a shared input hit L2.
 // LD_E / ST_E select whether consecutive threads walk elements (the pencil is
-// contiguous in memory) or pencils (pencils are adjacent in memory) when
-// moving data to and from the tile, so global accesses stay coalesced.
+// contiguous in memory) or pencils (pencils are adjacent in memory), so global
+// accesses stay coalesced.  Contiguous pencils are staged in the tile; adjacent
+// ones go straight from global memory to the registers of the first butterflies
+// and from those of the last ones back, so that the tile is written and read once
+// per pass boundary only (FP32 at 256 points: y passes 97 -> 84 and 62 -> 50 us,
+// z passes 68 -> 56 and 43 -> 34 us per launch of a 256^3 step, 3.5-3.9 -> 4.4-4.6
+// TB/s).
 #pragma once
 #include <type_traits>
 #include <utility>
@@ -29,21 +34,21 @@ template <class Op, class = void> struct HasKept : std::false_type {};
 template <class Op>
 struct HasKept<Op, std::void_t<decltype(std::declval<const Op&>().kept())>> : std::true_type {};
 
-template <typename T, class S, bool INV, class Op>
-__device__ __forceinline__ void pass_fft(const Op& op, C<T>* tile, const C<T>* tw) {
+template <typename T, class S, bool INV, bool DIN, bool DOUT, class Op, class Ld, class St>
+__device__ __forceinline__ void pass_fft(const Op& op, C<T>* tile, const C<T>* tw, Ld ld, St st) {
     if constexpr (HasKept<Op>::value && IsLF<T>::value) {   // one copy of the transform for double-float
-        if (op.kept() == kept23(S::L)) { pencil_fft_s<T, S, INV, true>(tile, tw); return; }
+        if (op.kept() == kept23(S::L)) { pencil_fft_io<T, S, INV, true, DIN, DOUT>(tile, tw, ld, st); return; }
     }
-    pencil_fft_s<T, S, INV, false>(tile, tw);
+    pencil_fft_io<T, S, INV, false, DIN, DOUT>(tile, tw, ld, st);
 }
 
-// Global -> tile: the P pencils of L elements starting at pencil f0, pencils
-// beyond npen zero.  Each thread loads its elements in groups of G into
+// Global -> tile: the P contiguous pencils of L elements starting at pencil f0,
+// pencils beyond npen zero.  Each thread loads its elements in groups of G into
 // registers before storing any of the group to shared memory, so a group's
 // global loads are in flight together (element-by-element load / store keeps
 // one load in flight per thread: the shared stores may not move above the
 // loads of generic pointers).
-template <typename T, int L, int P, int PS, int NT, bool LD_E, class Op>
+template <typename T, int L, int P, int PS, int NT, class Op>
 __device__ __forceinline__ void load_tile(const Op& op, C<T>* tile, int fld, int s, int f0, int npen) {
     constexpr int N = L * P;
     constexpr int NPT = (N + NT - 1) / NT;
@@ -57,8 +62,7 @@ __device__ __forceinline__ void load_tile(const Op& op, C<T>* tile, int fld, int
             const int idx = threadIdx.x + (i0 + i) * NT;
             v[i] = zero<T>();
             if (i0 + i < NPT && (N % NT == 0 || idx < N)) {
-                const int e = LD_E ? idx % L : idx / P;
-                const int p = LD_E ? idx / L : idx % P;
+                const int e = idx % L, p = idx / L;
                 if (f0 + p < npen) v[i] = op.load(fld, s, e, f0 + p);
             }
         }
@@ -66,8 +70,7 @@ __device__ __forceinline__ void load_tile(const Op& op, C<T>* tile, int fld, int
         for (int i = 0; i < G; i++) {
             const int idx = threadIdx.x + (i0 + i) * NT;
             if (i0 + i < NPT && (N % NT == 0 || idx < N)) {
-                const int e = LD_E ? idx % L : idx / P;
-                const int p = LD_E ? idx / L : idx % P;
+                const int e = idx % L, p = idx / L;
                 tile[e * PS + p] = v[i];
             }
         }
@@ -103,11 +106,7 @@ constexpr size_t pass_smem() {
     return S::template smem_bytes<T>() + (std::is_same<T, double>::value ? sizeof(unsigned) * FX_WORDS * S::P : 0);
 }
 
-// FP64: fixed-point transforms (fft_fixed.cuh).  Pencils that are adjacent in
-// memory go straight from global memory to the registers of the first
-// butterflies and from those of the last ones back, so that the tile is
-// written and read once per pass boundary only; contiguous pencils and real
-// rows are staged in the tile.
+// FP64: fixed-point transforms (fft_fixed.cuh).
 template <class S, bool INV, bool LD_E, bool ST_E, bool PRUNE, class Op>
 __device__ __forceinline__ void fx_pass_body(const Op& op, C<double>* tile, const int4* tw, unsigned* smax, int fld, int s,
                                              int f0, int npen) {
@@ -125,7 +124,7 @@ __device__ __forceinline__ void fx_pass_body(const Op& op, C<double>* tile, cons
         });
         __syncthreads();
     } else if constexpr (LD_E) {
-        load_tile<double, L, P, PS, NT, true>(op, tile, fld, s, f0, npen);
+        load_tile<double, L, P, PS, NT>(op, tile, fld, s, f0, npen);
         __syncthreads();
     }
     pencil_fx<S, INV, PRUNE, IN, OUT>(tile, tw, smax, ld, st);
@@ -166,17 +165,25 @@ __global__ void __launch_bounds__(S::NT, MB) k_pass(const Op op, int nfield) {
     } else {
         C<T>* tw = tile + L * PS;
         load_twiddles<T, L>(tw, op.tw);
-        load_tile<T, L, P, PS, NT, LD_E>(op, tile, fld, s, f0, npen);
-        __syncthreads();
-        pass_fft<T, S, INV>(op, tile, tw);
-        const int nst = op.nstore();
-        for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
-            const int e = ST_E ? idx % nst : idx / P;
-            const int p = ST_E ? idx / nst : idx % P;
-            const int f = f0 + p;
-            if (f >= npen) continue;
-            if constexpr (HasPut<Op>::value) op.put(fld, s, e, f, tile[e * PS + p]);
-            else op.store(fld, s, e, f, tile + p, PS);
+        constexpr bool DIN = !LD_E, DOUT = !ST_E;
+        if constexpr (LD_E) {
+            load_tile<T, L, P, PS, NT>(op, tile, fld, s, f0, npen);
+            __syncthreads();
+        }
+        const int f = f0 + threadIdx.x % P;
+        const auto ld = [&](int e) { return f < npen ? op.load(fld, s, e, f) : zero<T>(); };
+        const auto st = [&](int e, const C<T>& c) {
+            if constexpr (HasPut<Op>::value) { if (f < npen) op.put(fld, s, e, f, c); }
+        };
+        pass_fft<T, S, INV, DIN, DOUT>(op, tile, tw, ld, st);
+        if constexpr (ST_E) {
+            const int nst = op.nstore();
+            for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
+                const int e = idx % nst, p = idx / nst;
+                if (f0 + p >= npen) continue;
+                if constexpr (HasPut<Op>::value) op.put(fld, s, e, f0 + p, tile[e * PS + p]);
+                else op.store(fld, s, e, f0 + p, tile + p, PS);
+            }
         }
     }
 }
@@ -208,8 +215,9 @@ template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
 int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
     if constexpr (std::is_same<T, double>::value)
         return launch_pass_sched<T, FxS<L, INV>, INV, LD_E, ST_E, FxCfg<L>::MB>(op, npencil, nslow, nfield, st, "");
-    else
-        return launch_pass_sched<T, DefSched<L>, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st, "");
+    else   // FP32 inverse passes at 256 points: 5 blocks (48 registers) gain 4% on 4, forward ones spill
+        return launch_pass_sched<T, DefSched<L>, INV, LD_E, ST_E, (std::is_same<T, float>::value && L == 256 && INV ? 5 : 0)>(
+            op, npencil, nslow, nfield, st, "");
 }
 
 // Small-tile schedules (4 pencils, 16 threads each) for single-run 2D grids.
