@@ -241,8 +241,8 @@ int dd_fft_c2r(const dd_plan* p, int nfield, const void* const* k, double* const
 int dd_dealias(const dd_plan* p, void* k, void* stream) {
     DD_CHECK_ARG(p && k, "dd_dealias: null pointer");
     cudaStream_t st = (cudaStream_t)stream;
-    if (p->ndim == 3) DD_KT("dealias3", st, k_dealias3<<<ew_grid(p->g3.kcount()), 256, 0, st>>>(p->g3, (double2*)k));
-    else DD_KT("dealias2", st, k_dealias2<<<ew_grid(p->g2.kcount()), 256, 0, st>>>(p->g2, (double2*)k));
+    if (p->ndim == 3) DD_KT("dealias3", st, launch(k_dealias3, ew_grid(p->g3.kcount()), 256, 0, st, p->g3, (double2*)k));
+    else DD_KT("dealias2", st, launch(k_dealias2, ew_grid(p->g2.kcount()), 256, 0, st, p->g2, (double2*)k));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }

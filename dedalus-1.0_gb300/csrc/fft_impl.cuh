@@ -8,6 +8,7 @@ namespace dd {
 // -------------------------------------------------------- zero / dealias
 template <typename KT>
 __global__ void k_zero_nonkept3(Geo3 g, Ptrs k) {
+    grid_wait();
     using KV = typename Vec2<KT>::type;
     KV* K = (KV*)pick_ptr<DD_MAXF>(k.p, (int)blockIdx.y);
     const int64_t n = g.kcount();
@@ -20,6 +21,7 @@ __global__ void k_zero_nonkept3(Geo3 g, Ptrs k) {
 
 template <typename KT>
 __global__ void k_zero_nonkept2(Geo2 g, Ptrs k) {
+    grid_wait();
     using KV = typename Vec2<KT>::type;
     KV* K = (KV*)pick_ptr<DD_MAXF>(k.p, (int)blockIdx.y);
     const int64_t n0 = (int64_t)g.Kx * g.Ny, n = g.kcount();
@@ -29,6 +31,7 @@ __global__ void k_zero_nonkept2(Geo2 g, Ptrs k) {
 }
 
 static __global__ void k_dealias3(Geo3 g, double2* K) {
+    grid_wait();
     const int64_t n = g.kcount();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int kx = (int)(i % g.Nh);
@@ -39,6 +42,7 @@ static __global__ void k_dealias3(Geo3 g, double2* K) {
 }
 
 static __global__ void k_dealias2(Geo2 g, double2* K) {
+    grid_wait();
     const int64_t n = g.kcount();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int ky = (int)(i % g.Ny), kx = (int)(i / g.Ny);
@@ -123,7 +127,7 @@ int fft_r2c(const dd_plan* pl, int nf, const XT* const* x, void* const* k, void*
         OpZFwd3<T, double> c{g, w1c, ko, TwSel<T>::z(pl)};
         DD_TRY((launch_pass_len<T, false, false, false>(g.Nz, c, g.Kx, g.Ky, nf, st)));
         if (zero_nonkept) {
-            DD_KT("zero_nonkept3", st, k_zero_nonkept3<double><<<dim3(ew_grid(g.kcount()), nf), 256, 0, st>>>(g, ko));
+            DD_KT("zero_nonkept3", st, launch(k_zero_nonkept3<double>, dim3(ew_grid(g.kcount()), nf), 256, 0, st, g, ko));
             DD_LAUNCH_CHECK();
         }
     } else {
@@ -138,7 +142,7 @@ int fft_r2c(const dd_plan* pl, int nf, const XT* const* x, void* const* k, void*
         DD_TRY((launch_pass_len<T, false, false, true>(g.Ny, b, g.Kx, 1, nf, st)));
         const int64_t nz = g.kcount() - (int64_t)g.Kx * g.Ny;
         if (nz > 0 && zero_nonkept) {
-            DD_KT("zero_nonkept2", st, k_zero_nonkept2<double><<<dim3(ew_grid(nz), nf), 256, 0, st>>>(g, ko));
+            DD_KT("zero_nonkept2", st, launch(k_zero_nonkept2<double>, dim3(ew_grid(nz), nf), 256, 0, st, g, ko));
             DD_LAUNCH_CHECK();
         }
     }

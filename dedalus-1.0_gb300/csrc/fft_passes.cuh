@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(S::NT, MB) k_pass(const Op op, int nfield) {
         unsigned* smax = reinterpret_cast<unsigned*>(tw + L);
         fx_stage_twiddles<L, INV>(tw, op.tw);
         for (int i = threadIdx.x; i < FX_WORDS * P; i += NT) smax[i] = 0u;
+        grid_wait();
         if constexpr (HasKept<Op>::value) {
             if (op.kept() == kept23(L)) {
                 fx_pass_body<S, INV, LD_E, ST_E, true>(op, tile, tw, smax, fld, s, f0, npen);
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(S::NT, MB) k_pass(const Op op, int nfield) {
     } else {
         C<T>* tw = tile + L * PS;
         load_twiddles<T, L>(tw, op.tw);
+        grid_wait();
         constexpr bool DIN = !LD_E, DOUT = !ST_E;
         if constexpr (LD_E) {
             load_tile<T, L, P, PS, NT>(op, tile, fld, s, f0, npen);
@@ -202,7 +204,7 @@ int launch_pass_sched(const Op& op, int npencil, int nslow, int nfield, cudaStre
     }
     dim3 grid(cdiv(npencil, S::P) * nfield, nslow > 65535 ? 65535 : nslow, nslow > 65535 ? nslow / 65535 : 1);
     static const std::string label = std::string(Op::name) + "_" + std::to_string(S::L) + tag + PrecName<T>::s;
-    DD_KT(label.c_str(), st, kern<<<grid, S::NT, smem, st>>>(op, nfield));
+    DD_KT(label.c_str(), st, launch(kern, grid, S::NT, smem, st, op, nfield));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }

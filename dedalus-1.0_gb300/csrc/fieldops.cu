@@ -11,6 +11,7 @@ namespace dd {
 // axis: 0 = x, 1 = y, 2 = z (component names, not storage order).
 __global__ void k_deriv(int ndim, int n0, int n1, int n2, int axis, const double* kx, const double* ky,
                         const double* kz, const double2* in, double2* out) {
+    grid_wait();
     const int64_t n = (int64_t)n0 * n1 * n2;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double k;
@@ -32,6 +33,7 @@ __global__ void k_deriv(int ndim, int n0, int n1, int n2, int axis, const double
 // numpy forms `comp = kd / 6.` and `comp += kd / 3.` (time_step.py:435, 452),
 // numpy dividing by multiplying with the reciprocal.
 __global__ void k_scale_add(const double2* x, double2* y, double w, int accumulate, int64_t n) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double2 a = x[i];
         double2 r = make_double2(__dmul_rn(a.x, w), __dmul_rn(a.y, w));
@@ -85,7 +87,7 @@ int dd_deriv(const dd_plan* p, int axis, const void* k_in, void* k_out, void* st
     else { n0 = p->g2.Nh; n1 = p->g2.Ny; n2 = 1; }
     const int64_t n = (int64_t)n0 * n1 * n2;
     DD_KT("deriv", (cudaStream_t)stream,
-          k_deriv<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(p->ndim, n0, n1, n2, axis, p->kx, p->ky, p->kz,
+          launch(k_deriv, grid_for(n), 256, 0, (cudaStream_t)stream, p->ndim, n0, n1, n2, axis, p->kx, p->ky, p->kz,
                                                                  (const double2*)k_in, (double2*)k_out));
     DD_LAUNCH_CHECK();
     return DD_OK;
@@ -95,7 +97,7 @@ int dd_scale_add(const void* x, void* y, double w, int accumulate, int64_t n, vo
     DD_CHECK_ARG(x && y && n >= 0, "dd_scale_add: bad arguments");
     if (n == 0) return DD_OK;
     DD_KT("scale_add", (cudaStream_t)stream,
-          k_scale_add<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const double2*)x, (double2*)y, w, accumulate, n));
+          launch(k_scale_add, grid_for(n), 256, 0, (cudaStream_t)stream, (const double2*)x, (double2*)y, w, accumulate, n));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }

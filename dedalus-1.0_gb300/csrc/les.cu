@@ -36,6 +36,7 @@ __device__ __forceinline__ double2 les_ik(double2 a, double k) { return make_dou
 // gk[3 a + j] = i k_j y_a on the kept modes (full layout out).
 template <bool COMPACT>
 __global__ void k_les_grad9(Geo3 g, const double* kx, const double* ky, const double* kz, CPtrs y, Ptrs gk) {
+    grid_wait();
     const int64_t n = (int64_t)g.Ky * g.Kz * g.Kx;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int ky_i, kz_i, ix;
@@ -113,6 +114,7 @@ __device__ __forceinline__ void les_act(const float c[4], const float* bias, uin
 template <typename GT, typename TT>
 __global__ void __launch_bounds__(32 * LES_WARPS) k_les_mlp(CPtrs gx, Ptrs tau, int64_t npts, const bf16* wb,
                                                             const float* p, const float* norm, double delta) {
+    grid_wait();
     __shared__ __align__(16) LesMlpSmem s;
     for (int i = threadIdx.x; i < MLP_H * MLP_IN; i += blockDim.x)
         s.w1[(i / MLP_IN) * LDI + i % MLP_IN] = wb[BOFF_W1 + i];
@@ -238,6 +240,7 @@ __device__ __forceinline__ double les_weight(double kk, const double* sw, int ns
 // order xx, yy, zz, xy, xz, yz; nc compact complex128; w from les_weight.
 __global__ void k_les_add(Geo3 g, const double* kx, const double* ky, const double* kz, CPtrs tk, Ptrs nc,
                           double lo, double hi, const double* sw, int nsw) {
+    grid_wait();
     const int64_t n = (int64_t)g.Ky * g.Kz * g.Kx;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int ky_i, kz_i, ix;
@@ -420,8 +423,8 @@ static int les_grads(const dd_plan* p, int prec, bool compact, const void* const
     for (int a = 0; a < 3; a++) yc.p[a] = y[a];
     for (int f = 0; f < 9; f++) gk.p[f] = w.gk[f];
     const unsigned nb = les_grid((int64_t)g.Ky * g.Kz * g.Kx);
-    if (compact) DD_KT("les_grad9", st, k_les_grad9<true><<<nb, 256, 0, st>>>(g, p->kx, p->ky, p->kz, yc, gk));
-    else DD_KT("les_grad9", st, k_les_grad9<false><<<nb, 256, 0, st>>>(g, p->kx, p->ky, p->kz, yc, gk));
+    if (compact) DD_KT("les_grad9", st, launch(k_les_grad9<true>, nb, 256, 0, st, g, p->kx, p->ky, p->kz, yc, gk));
+    else DD_KT("les_grad9", st, launch(k_les_grad9<false>, nb, 256, 0, st, g, p->kx, p->ky, p->kz, yc, gk));
     DD_LAUNCH_CHECK();
     const void* kin[9];
     for (int f = 0; f < 9; f++) kin[f] = w.gk[f];
@@ -451,7 +454,7 @@ static int les_mlp(const dd_plan* p, const dd_closure* cl, const GT* const* gxi,
     const int64_t need = (npts + 16 * LES_WARPS - 1) / (16 * LES_WARPS);
     const unsigned nb = (unsigned)(need < nres ? (need < 1 ? 1 : need) : nres);
     DD_KT("les_mlp", st,
-          (k_les_mlp<GT, TT><<<nb, 32 * LES_WARPS, 0, st>>>(gx, t, npts, (const bf16*)cl->wbf16, cl->params, cl->norm,
+          (launch(k_les_mlp<GT, TT>, nb, 32 * LES_WARPS, 0, st, gx, t, npts, (const bf16*)cl->wbf16, cl->params, cl->norm,
                                                             cl->delta)));
     DD_LAUNCH_CHECK();
     return DD_OK;
@@ -480,7 +483,7 @@ int les_closure_add(const dd_plan* p, const LesHook& h, int prec, bool compact, 
     for (int c = 0; c < 6; c++) tk.p[c] = w.gk[c];
     for (int a = 0; a < 3; a++) n.p[a] = nc[a];
     DD_KT("les_add", st,
-          k_les_add<<<les_grid((int64_t)g.Ky * g.Kz * g.Kx), 256, 0, st>>>(g, p->kx, p->ky, p->kz, tk, n,
+          launch(k_les_add, les_grid((int64_t)g.Ky * g.Kz * g.Kx), 256, 0, st, g, p->kx, p->ky, p->kz, tk, n,
                                                                           h.cl->band_lo, h.cl->band_hi,
                                                                           h.cl->shell_w, h.cl->n_shell));
     DD_LAUNCH_CHECK();

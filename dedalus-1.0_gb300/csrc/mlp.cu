@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
                                                           const int64_t* __restrict__ idx, int64_t n,
                                                           const bf16* wb, const float* p, float scale,
                                                           float* __restrict__ part) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char mlp_smem[];
     MlpSmem& s = *reinterpret_cast<MlpSmem*>(mlp_smem);
     mlp_load_weights(s, wb, p);
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
 
 // grad[j] = sum_b part[b][j] in block order; loss[0] = sum_b part[b][NPARAM].
 __global__ void k_mlp_reduce(const float* __restrict__ part, int nblk, float* grad, float* loss) {
+    grid_wait();
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= MLP_NPARAM; j += gridDim.x * blockDim.x) {
         float t = 0.f;
         for (int b = 0; b < nblk; b++) t += part[(int64_t)b * MLP_PSTRIDE + j];
@@ -250,6 +252,7 @@ __global__ void k_mlp_pack(const float* p, bf16* wb) {
 // p -= lr (m / bc1) / (sqrt(v / bc2) + eps) with bc = 1 - beta^step.
 __global__ void k_mlp_adam(float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
                            float bc1, float bc2) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < MLP_NPARAM; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -334,10 +337,10 @@ int dd_mlp_grad(const void* X, const float* T, const int64_t* idx, int64_t n, in
     const float scale = 2.0f / ((float)n_total * (float)MLP_NOUT);
     float* part = (float*)work;
     DD_KT("mlp_grad", st,
-          k_mlp_grad<<<nb, MLP_THREADS, sizeof(MlpSmem), st>>>((const bf16*)X, T, idx, n, (const bf16*)wbf16, params,
+          launch(k_mlp_grad, nb, MLP_THREADS, sizeof(MlpSmem), st, (const bf16*)X, T, idx, n, (const bf16*)wbf16, params,
                                                                 scale, part));
     DD_LAUNCH_CHECK();
-    DD_KT("mlp_reduce", st, k_mlp_reduce<<<ew_blocks(MLP_NPARAM + 1, 256), 256, 0, st>>>(part, nb, grad, loss));
+    DD_KT("mlp_reduce", st, launch(k_mlp_reduce, ew_blocks(MLP_NPARAM + 1, 256), 256, 0, st, part, nb, grad, loss));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -348,7 +351,7 @@ int dd_mlp_adam(float* params, const float* grad, float* m, float* v, int step, 
     cudaStream_t st = (cudaStream_t)stream;
     const float bc1 = 1.f - powf(beta1, (float)step), bc2 = 1.f - powf(beta2, (float)step);
     DD_KT("mlp_adam", st,
-          k_mlp_adam<<<ew_blocks(MLP_NPARAM, 256), 256, 0, st>>>(params, grad, m, v, lr, beta1, beta2, eps, bc1, bc2));
+          launch(k_mlp_adam, ew_blocks(MLP_NPARAM, 256), 256, 0, st, params, grad, m, v, lr, beta1, beta2, eps, bc1, bc2));
     DD_LAUNCH_CHECK();
     return dd_mlp_pack(params, wbf16, stream);
 }

@@ -67,6 +67,7 @@ __device__ __forceinline__ void phis2(const Stage2Args& a, int c, int q, double 
 // parameters so that the per-field loop unrolls with static indices.
 template <int NF, int MODE, bool DIV>
 __global__ void k_stage2(Stage2Args a) {
+    grid_wait();
     const Geo2& g = a.g;
     const int per = g.Kx * g.Ky;
     const int64_t n = (int64_t)per * a.nrun;
@@ -146,6 +147,7 @@ __global__ void k_stage2(Stage2Args a) {
 // it to f0 y in FP64 (the state stays FP64).
 template <int NF, int MODE>
 __global__ void k_stage2_lo(Stage2Args a) {
+    grid_wait();
     static_assert(MODE == 1 || MODE == 2, "RK2mid stages only");
     const Geo2& g = a.g;
     const int per = g.Kx * g.Ky;
@@ -239,18 +241,18 @@ __global__ void k_stage2_lo(Stage2Args a) {
 
 template <int MODE>
 static int launch_stage2_lo(const Stage2Args& a, unsigned nb, cudaStream_t st) {
-    if (a.phys == PHYS_HYDRO_DIV) DD_KT("rk2mid_stage2d_lo", st, k_stage2_lo<2, MODE><<<nb, 256, 0, st>>>(a));
-    else DD_KT("rk2mid_stage2d_lo", st, k_stage2_lo<3, MODE><<<nb, 256, 0, st>>>(a));
+    if (a.phys == PHYS_HYDRO_DIV) DD_KT("rk2mid_stage2d_lo", st, launch(k_stage2_lo<2, MODE>, nb, 256, 0, st, a));
+    else DD_KT("rk2mid_stage2d_lo", st, launch(k_stage2_lo<3, MODE>, nb, 256, 0, st, a));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
 
 template <int MODE>
 static int launch_stage2(const Stage2Args& a, unsigned nb, const char* label, cudaStream_t st) {
-    if (a.phys == PHYS_HYDRO) DD_KT(label, st, k_stage2<2, MODE, false><<<nb, 256, 0, st>>>(a));
-    else if (a.phys == PHYS_BOUSS) DD_KT(label, st, k_stage2<3, MODE, false><<<nb, 256, 0, st>>>(a));
-    else if (a.phys == PHYS_HYDRO_DIV) DD_KT(label, st, k_stage2<2, MODE, true><<<nb, 256, 0, st>>>(a));
-    else DD_KT(label, st, k_stage2<3, MODE, true><<<nb, 256, 0, st>>>(a));
+    if (a.phys == PHYS_HYDRO) DD_KT(label, st, launch(k_stage2<2, MODE, false>, nb, 256, 0, st, a));
+    else if (a.phys == PHYS_BOUSS) DD_KT(label, st, launch(k_stage2<3, MODE, false>, nb, 256, 0, st, a));
+    else if (a.phys == PHYS_HYDRO_DIV) DD_KT(label, st, launch(k_stage2<2, MODE, true>, nb, 256, 0, st, a));
+    else DD_KT(label, st, launch(k_stage2<3, MODE, true>, nb, 256, 0, st, a));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -258,6 +260,7 @@ static int launch_stage2(const Stage2Args& a, unsigned nb, const char* label, cu
 // Non-kept modes see no forcing: RK2mid gives y <- etd2rk2(y, 0, 0, dt) = f0 y.
 __global__ void k_decay_nonkept2(Geo2 g, Ptrs y, int64_t y_rs, int nf, int nrun, const double* kx,
                                  const double* ky, Stage2Args a) {
+    grid_wait();
     const int64_t per = g.kcount(), n = per * nrun;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int run = (int)(i / per);
@@ -279,6 +282,7 @@ __global__ void k_decay_nonkept2(Geo2 g, Ptrs y, int64_t y_rs, int nf, int nrun,
 }
 
 __global__ void k_zero_nonkept2_all(Geo2 g, Ptrs k, int64_t rs, int nrun) {
+    grid_wait();
     double2* K = (double2*)pick_ptr<DD_MAXF>(k.p, (int)blockIdx.y);
     const int64_t per = g.kcount(), n = per * nrun;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -293,6 +297,7 @@ __global__ void k_zero_nonkept2_all(Geo2 g, Ptrs k, int64_t rs, int nrun) {
 // out[0] += |k . u|^2, out[1] += |k|^2 |u|^2 (block partials, one atomic per block).
 __global__ void __launch_bounds__(256) k_div_sums2(Geo2 g, const double* kx, const double* ky, const double2* ux,
                                                     const double2* uy, int64_t rs, int nrun, double* out) {
+    grid_wait();
     __shared__ double r0[256], r1[256];
     const int per = g.Kx * g.Ky;
     const int64_t n = (int64_t)per * nrun;
@@ -418,7 +423,7 @@ int dd_rhs2d(const dd_plan* p, int phys, const double* params, int nrun, const v
     if (zero_nonkept) {
         Ptrs d{};
         for (int c = 0; c < nf; c++) d.p[c] = deriv[c];
-        DD_KT("zero_nonkept2", st, k_zero_nonkept2_all<<<dim3(ew_grid2(p->g2.kcount() * nrun), nf), 256, 0, st>>>(
+        DD_KT("zero_nonkept2", st, launch(k_zero_nonkept2_all, dim3(ew_grid2(p->g2.kcount() * nrun), nf), 256, 0, st, 
                                        p->g2, d, deriv_rs, nrun));
         DD_LAUNCH_CHECK();
     }
@@ -473,7 +478,7 @@ int dd_rk2mid_step2d(const dd_plan* p, int phys, const double* params, int nrun,
     if (lo) DD_TRY(launch_stage2_lo<2>(a, nb, st));
     else DD_TRY(launch_stage2<2>(a, nb, "rk2mid_stage2d", st));
     if (!nonkept_flag || *nonkept_flag) {
-        DD_KT("decay_nonkept2", st, k_decay_nonkept2<<<ew_grid2(p->g2.kcount() * nrun), 256, 0, st>>>(
+        DD_KT("decay_nonkept2", st, launch(k_decay_nonkept2, ew_grid2(p->g2.kcount() * nrun), 256, 0, st, 
                                         p->g2, a.y, state_rs, nf, nrun, p->kx, p->ky, a));
         DD_LAUNCH_CHECK();
     }
@@ -489,7 +494,7 @@ int dd_divergence_sums2d(const dd_plan* p, int nrun, const void* ux, const void*
     const Geo2& g = p->g2;
     const int64_t n = (int64_t)g.Kx * g.Ky * nrun;
     const unsigned nb = (unsigned)std::min<int64_t>((n + 255) / 256, 152 * 4);
-    DD_KT("div_sums2", st, k_div_sums2<<<nb, 256, 0, st>>>(g, p->kx, p->ky, (const double2*)ux, (const double2*)uy,
+    DD_KT("div_sums2", st, launch(k_div_sums2, nb, 256, 0, st, g, p->kx, p->ky, (const double2*)ux, (const double2*)uy,
                                                           run_stride, nrun, out));
     DD_LAUNCH_CHECK();
     return DD_OK;

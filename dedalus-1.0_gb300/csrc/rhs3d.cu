@@ -113,6 +113,7 @@ __device__ __forceinline__ void rhs_at(const CPtrs& nc, int64_t i, double kxv, d
 
 template <int PH>
 __global__ void k_project_to_deriv3(ProjArgs a, CPtrs nc, Ptrs deriv) {
+    grid_wait();
     const Geo3& g = a.g;
     const int64_t n = (int64_t)g.Ky * g.Kz * g.Kx;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -163,6 +164,7 @@ __device__ __forceinline__ void phis_for(const RK4Args& a, int grp, int q, doubl
 
 template <int PH>
 __global__ void k_rk4_stage3(RK4Args a) {
+    grid_wait();
     const Geo3& g = a.pa.g;
     constexpr int NF = Phys3<PH>::NF, NG = Phys3<PH>::NG;
     const int n = g.Ky * g.Kz * g.Kx;      // < 2^31 for every supported grid
@@ -216,6 +218,7 @@ __device__ __forceinline__ float2 fderiv(float2 a, float k) { return make_float2
 
 template <int PH>
 __global__ void k_rk4_stage3_lo(RK4Args a) {
+    grid_wait();
     static_assert(PH == P3_HYDRO_DIV || PH == P3_MHD_DIV, "low-storage stages are for the divergence forms");
     const Geo3& g = a.pa.g;
     constexpr int NF = Phys3<PH>::NF, NG = Phys3<PH>::NG;
@@ -314,6 +317,7 @@ __global__ void k_rk4_stage3_lo(RK4Args a) {
 
 // Non-kept modes of the state see no nonlinear forcing: y <- etd1(y, 0, dt).
 __global__ void k_decay_nonkept3(RK4Args a, int ncomp) {
+    grid_wait();
     const Geo3& g = a.pa.g;
     const int64_t n = g.kcount();
     const int c = blockIdx.y;
@@ -357,6 +361,7 @@ __global__ void k_any_nonkept3(Geo3 g, CPtrs y, int ncomp, int* flag) {
 
 // Zero every non-kept entry of full-layout arrays (grid.y = component).
 __global__ void k_dealias3_all(Geo3 g, Ptrs k) {
+    grid_wait();
     double2* K = (double2*)pick_ptr<DD_MAXF>(k.p, (int)blockIdx.y);
     const int64_t n = g.kcount();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -371,6 +376,7 @@ __global__ void k_dealias3_all(Geo3 g, Ptrs k) {
 // out[1] += |k|^2 |u|^2 (block partials, then one atomic add per block).
 __global__ void __launch_bounds__(256) k_div_sums3(Geo3 g, const double* kx, const double* ky, const double* kz,
                                                     CPtrs u, double* out) {
+    grid_wait();
     __shared__ double r0[256], r1[256];
     const int n = g.Ky * g.Kz * g.Kx;      // < 2^31 for every supported grid
     double s0 = 0., s1 = 0.;
@@ -468,10 +474,10 @@ static int rhs3(const dd_plan* p, const double* params, const void* const* u, vo
         DD_TRY(les_closure_add(p, *les, prec, false, u, ncp, st));
     }
     if (zero_nonkept) {
-        DD_KT("zero_nonkept3", st, k_dealias3_all<<<dim3(ew_grid(g.kcount()), P::NF), 256, 0, st>>>(g, d));
+        DD_KT("zero_nonkept3", st, launch(k_dealias3_all, dim3(ew_grid(g.kcount()), P::NF), 256, 0, st, g, d));
         DD_LAUNCH_CHECK();
     }
-    DD_KT("project3", st, k_project_to_deriv3<PH><<<ew_grid((int64_t)g.Ky * g.Kz * g.Kx), 256, 0, st>>>(pa, nc, d));
+    DD_KT("project3", st, launch(k_project_to_deriv3<PH>, ew_grid((int64_t)g.Ky * g.Kz * g.Kx), 256, 0, st, pa, nc, d));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -515,7 +521,7 @@ static int rk4_3(const dd_plan* p, const double* params, void* const* u, const d
                 a.stage = s; a.h = hs[s - 1]; a.w = ws[s - 1];
                 for (int grp = 0; grp < P::NG; grp++)
                     a.tab[grp] = intk ? (const double4*)(s <= 2 ? tab_half[grp] : tab_full[grp]) : nullptr;
-                DD_KT("rk4_stage3_lo", st, k_rk4_stage3_lo<PH><<<nb, 256, 0, st>>>(a));
+                DD_KT("rk4_stage3_lo", st, launch(k_rk4_stage3_lo<PH>, nb, 256, 0, st, a));
                 DD_LAUNCH_CHECK();
                 continue;
             }
@@ -528,11 +534,11 @@ static int rk4_3(const dd_plan* p, const double* params, void* const* u, const d
         a.stage = s; a.h = hs[s - 1]; a.w = ws[s - 1];
         for (int grp = 0; grp < P::NG; grp++)
             a.tab[grp] = intk ? (const double4*)(s <= 2 ? tab_half[grp] : tab_full[grp]) : nullptr;
-        DD_KT("rk4_stage3", st, k_rk4_stage3<PH><<<nb, 256, 0, st>>>(a));
+        DD_KT("rk4_stage3", st, launch(k_rk4_stage3<PH>, nb, 256, 0, st, a));
         DD_LAUNCH_CHECK();
     }
     if (!nonkept_flag || *nonkept_flag) {
-        DD_KT("decay_nonkept3", st, k_decay_nonkept3<<<dim3(ew_grid(g.kcount()), P::NF), 256, 0, st>>>(a, P::NF));
+        DD_KT("decay_nonkept3", st, launch(k_decay_nonkept3, dim3(ew_grid(g.kcount()), P::NF), 256, 0, st, a, P::NF));
         DD_LAUNCH_CHECK();
     }
     return DD_OK;
@@ -686,7 +692,7 @@ int dd_divergence_sums(const dd_plan* p, const void* const* u, double* out, void
     const Geo3& g = p->g3;
     const int64_t nk = (int64_t)g.Ky * g.Kz * g.Kx;
     const unsigned nb = (unsigned)std::min<int64_t>((nk + 255) / 256, 152 * 4);
-    DD_KT("div_sums3", st, k_div_sums3<<<nb, 256, 0, st>>>(g, p->kx, p->ky, p->kz, uc, out));
+    DD_KT("div_sums3", st, launch(k_div_sums3, nb, 256, 0, st, g, p->kx, p->ky, p->kz, uc, out));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }

@@ -157,6 +157,7 @@ __global__ void k_shear_zero_cols3(Geo3 g, Ptrs k) {
 
 // In-place 2/3 rule with the sheared k_y (dealias_cy_{2d,3d}.pyx, sheared branch).
 __global__ void k_shear_dealias(int ndim, Geo3 g3, Geo2 g2, const double* kys, double cut, Ptrs k) {
+    grid_wait();
     double2* K = (double2*)k.p[blockIdx.y];
     const int64_t n = ndim == 3 ? g3.kcount() : g2.kcount();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -177,6 +178,7 @@ __global__ void k_shear_dealias(int ndim, Geo3 g3, Geo2 g2, const double* kys, d
 // out = in * (1j * k) with k the sheared k_y table (broadcast over kz in 3D):
 // numpy's complex product ((-b k), a k), as the static dd_deriv.
 __global__ void k_shear_deriv_y(int ndim, Geo3 g3, Geo2 g2, const double* kys, const double2* in, double2* out) {
+    grid_wait();
     const int64_t n = ndim == 3 ? g3.kcount() : g2.kcount();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double k;
@@ -198,6 +200,7 @@ __global__ void k_shear_deriv_y(int ndim, Geo3 g3, Geo2 g2, const double* kys, c
 // operation is rounded separately, as numpy's elementwise expressions are.
 __global__ void k_kreal(int64_t n, const double2* in, const double* r, double w, int mode, int accumulate,
                         double2* out) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double2 a = in[i];
         const double f = mode == 0 ? __ddiv_rn(1.0, r[i]) : r[i];
@@ -211,6 +214,7 @@ __global__ void k_kreal(int64_t n, const double2* in, const double* r, double w,
 // Grid points: out = (accumulate ? out : 0) + (a * b) * w (b == NULL: a * w),
 // each operation rounded separately.
 __global__ void k_xfma(int64_t n, const double* a, const double* b, double w, int accumulate, double* out) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double v = b ? __dmul_rn(a[i], b[i]) : a[i];
         if (w != 1.) v = __dmul_rn(v, w);
@@ -293,7 +297,7 @@ int dd_shear_r2c(const dd_plan* p, int nfield, const double* const* x, void* con
         DD_TRY((launch_pass_len<double, false, false, true>(g.Ny, b, g.Kx, 1, nfield, st)));
         const int64_t nz = g.kcount() - (int64_t)g.Kx * g.Ny;
         if (nz > 0) {
-            DD_KT("zero_nonkept2", st, k_zero_nonkept2<double><<<dim3(sh_grid(nz), nfield), 256, 0, st>>>(g, ko));
+            DD_KT("zero_nonkept2", st, launch(k_zero_nonkept2<double>, dim3(sh_grid(nz), nfield), 256, 0, st, g, ko));
             DD_LAUNCH_CHECK();
         }
     }
@@ -353,7 +357,7 @@ int dd_shear_dealias(const dd_plan* p, int nfield, void* const* k, const double*
     const int64_t n = p->ndim == 3 ? p->g3.kcount() : p->g2.kcount();
     cudaStream_t st = (cudaStream_t)stream;
     DD_KT("shear_dealias", st,
-          k_shear_dealias<<<dim3(sh_grid(n), nfield), 256, 0, st>>>(p->ndim, p->g3, p->g2, kys, cut, kp));
+          launch(k_shear_dealias, dim3(sh_grid(n), nfield), 256, 0, st, p->ndim, p->g3, p->g2, kys, cut, kp));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -363,7 +367,7 @@ int dd_shear_deriv_y(const dd_plan* p, const double* kys, const void* k_in, void
     const int64_t n = p->ndim == 3 ? p->g3.kcount() : p->g2.kcount();
     cudaStream_t st = (cudaStream_t)stream;
     DD_KT("shear_deriv_y", st,
-          k_shear_deriv_y<<<sh_grid(n), 256, 0, st>>>(p->ndim, p->g3, p->g2, kys, (const double2*)k_in,
+          launch(k_shear_deriv_y, sh_grid(n), 256, 0, st, p->ndim, p->g3, p->g2, kys, (const double2*)k_in,
                                                        (double2*)k_out));
     DD_LAUNCH_CHECK();
     return DD_OK;
@@ -376,7 +380,7 @@ int dd_kspace_real(int64_t n, const void* in, const double* r, double w, int mod
     if (n == 0) return DD_OK;
     cudaStream_t st = (cudaStream_t)stream;
     DD_KT("kspace_real", st,
-          k_kreal<<<sh_grid(n), 256, 0, st>>>(n, (const double2*)in, r, w, mode, accumulate, (double2*)out));
+          launch(k_kreal, sh_grid(n), 256, 0, st, n, (const double2*)in, r, w, mode, accumulate, (double2*)out));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -385,7 +389,7 @@ int dd_xspace_fma(int64_t n, const double* a, const double* b, double w, int acc
     DD_CHECK_ARG(a && out && n >= 0, "dd_xspace_fma: bad arguments");
     if (n == 0) return DD_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    DD_KT("xspace_fma", st, k_xfma<<<sh_grid(n), 256, 0, st>>>(n, a, b, w, accumulate, out));
+    DD_KT("xspace_fma", st, launch(k_xfma, sh_grid(n), 256, 0, st, n, a, b, w, accumulate, out));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }

@@ -8,6 +8,7 @@ namespace dd {
 
 __global__ void k_euler(const double2* __restrict__ s, double2* o, const double2* __restrict__ d,
                         double dt, int64_t n) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double2 a = s[i], b = d[i];
         double2 r;
@@ -20,6 +21,7 @@ __global__ void k_euler(const double2* __restrict__ s, double2* o, const double2
 template <int NDIM>
 __global__ void k_etd1(const double2* s, double2* o, const double2* __restrict__ d,
                        const double* __restrict__ intf, double dt, int64_t n) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double Z = rmul(intf[i], dt);
         double f0 = 1., f1 = 1., f2 = 0.5;
@@ -32,6 +34,7 @@ template <int NDIM>
 __global__ void k_etd2rk1(const double2* s, double2* o, const double2* __restrict__ d1,
                           const double2* __restrict__ d2, const double* __restrict__ intf,
                           double dt, int64_t n) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double Z = rmul(intf[i], dt);
         double f0 = 1., f1 = 1., f2 = 0.5;
@@ -44,6 +47,7 @@ template <int NDIM>
 __global__ void k_etd2rk2(const double2* s, double2* o, const double2* __restrict__ d1,
                           const double2* __restrict__ d2, const double* __restrict__ intf,
                           double dt, int64_t n) {
+    grid_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double Z = rmul(intf[i], dt);
         double f0 = 1., f1 = 1., f2 = 0.5;
@@ -85,7 +89,7 @@ int dd_euler(const void* start, void* output, const void* deriv, double dt, int6
     DD_CHECK_ARG(n >= 0, "dd_euler: negative size");
     if (n == 0) return DD_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    DD_KT("euler", st, k_euler<<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output,
+    DD_KT("euler", st, launch(k_euler, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output,
                                                              (const double2*)deriv, dt, n));
     DD_LAUNCH_CHECK();
     return DD_OK;
@@ -99,9 +103,9 @@ int dd_etd1(int ndim, const void* start, void* output, const void* deriv, const 
     if (n == 0) return DD_OK;
     cudaStream_t st = (cudaStream_t)stream;
     if (ndim == 2)
-        DD_KT("etd12", st, k_etd1<2><<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output, (const double2*)deriv, intfactor, dt, n));
+        DD_KT("etd12", st, launch(k_etd1<2>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv, intfactor, dt, n));
     else
-        DD_KT("etd13", st, k_etd1<3><<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output, (const double2*)deriv, intfactor, dt, n));
+        DD_KT("etd13", st, launch(k_etd1<3>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv, intfactor, dt, n));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -114,10 +118,10 @@ int dd_etd2rk1(int ndim, const void* start, void* output, const void* deriv1, co
     if (n == 0) return DD_OK;
     cudaStream_t st = (cudaStream_t)stream;
     if (ndim == 2)
-        DD_KT("etd2rk12", st, k_etd2rk1<2><<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output, (const double2*)deriv1,
+        DD_KT("etd2rk12", st, launch(k_etd2rk1<2>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv1,
                                                    (const double2*)deriv2, intfactor, dt, n));
     else
-        DD_KT("etd2rk13", st, k_etd2rk1<3><<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output, (const double2*)deriv1,
+        DD_KT("etd2rk13", st, launch(k_etd2rk1<3>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv1,
                                                    (const double2*)deriv2, intfactor, dt, n));
     DD_LAUNCH_CHECK();
     return DD_OK;
@@ -131,10 +135,10 @@ int dd_etd2rk2(int ndim, const void* start, void* output, const void* deriv1, co
     if (n == 0) return DD_OK;
     cudaStream_t st = (cudaStream_t)stream;
     if (ndim == 2)
-        DD_KT("etd2rk22", st, k_etd2rk2<2><<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output, (const double2*)deriv1,
+        DD_KT("etd2rk22", st, launch(k_etd2rk2<2>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv1,
                                                    (const double2*)deriv2, intfactor, dt, n));
     else
-        DD_KT("etd2rk23", st, k_etd2rk2<3><<<ew_blocks(n), 256, 0, st>>>((const double2*)start, (double2*)output, (const double2*)deriv1,
+        DD_KT("etd2rk23", st, launch(k_etd2rk2<3>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv1,
                                                    (const double2*)deriv2, intfactor, dt, n));
     DD_LAUNCH_CHECK();
     return DD_OK;

@@ -172,6 +172,7 @@ k_x_prod(int nrows, int Kx, CPtrs win, Ptrs wout, int64_t in_rs, int64_t out_rs,
     constexpr size_t TA = (size_t)SI::span, TB = (size_t)SF::span;
     C<T>* tw = tile + (TA > TB ? TA : TB);
     load_twiddles<T, L>(tw, gtw);
+    grid_wait();
     const int row0 = blockIdx.x * Q;
     const int nr = min(Q, nrows - row0);
     const int64_t ib = blockIdx.y * in_rs, ob = blockIdx.y * out_rs;  // run (batch) offsets
@@ -465,6 +466,7 @@ k_x_prod_fx(int nrows, int Kx, CPtrs win, Ptrs wout, int64_t in_rs, int64_t out_
     fx_stage_twiddles<L, true>(twi, gtw);
     fx_stage_twiddles<L, false>(twf, gtw);
     for (int i = threadIdx.x; i < FX_WORDS * (CC::SI::P + CC::SF::P); i += NT) smi[i] = 0u;
+    grid_wait();
     const int64_t ib = blockIdx.y * in_rs, ob = blockIdx.y * out_rs;  // run (batch) offsets
     if (Kx - 1 == kept23(L)) x_prod_fx_body<L, true>(nrows, Kx, win, wout, ib, ob, tile, twi, twf, smi, smf, sexp, smul, op);
     else x_prod_fx_body<L, false>(nrows, Kx, win, wout, ib, ob, tile, twi, twf, smi, smf, sexp, smul, op);
@@ -483,7 +485,7 @@ int launch_x_prod(const char* name, int nrows, int Kx, const CPtrs& win, const P
         double smul;
         fx_split_scale(scale, sexp, smul);
         DD_KT(label.c_str(), st,
-              k_x_prod_fx<L, Op><<<dim3(cdiv(nrows, CC::Q), nrun), CC::NT, smem, st>>>(nrows, Kx, win, wout, in_rs, out_rs, tw,
+              launch(k_x_prod_fx<L, Op>, dim3(cdiv(nrows, CC::Q), nrun), CC::NT, smem, st, nrows, Kx, win, wout, in_rs, out_rs, tw,
                                                                                        sexp, smul, op));
         DD_LAUNCH_CHECK();
         return DD_OK;
@@ -493,7 +495,7 @@ int launch_x_prod(const char* name, int nrows, int Kx, const CPtrs& win, const P
     DD_TRY(ensure_smem((const void*)k_x_prod<T, L, Op>, smem, configured));
     static const std::string label = std::string(name) + "_" + std::to_string(L) + PrecName<T>::s;
     DD_KT(label.c_str(), st,
-          k_x_prod<T, L, Op><<<dim3(cdiv(nrows, CC::Q), nrun), CC::NT, smem, st>>>(nrows, Kx, win, wout, in_rs, out_rs,
+          launch(k_x_prod<T, L, Op>, dim3(cdiv(nrows, CC::Q), nrun), CC::NT, smem, st, nrows, Kx, win, wout, in_rs, out_rs,
                                                                                   tw, scale, op));
     DD_LAUNCH_CHECK();
     return DD_OK;
