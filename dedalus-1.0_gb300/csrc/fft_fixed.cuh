@@ -299,6 +299,15 @@ __device__ __forceinline__ bool fx_has(int b, int jt) {
     return NB % S::TPP == 0 || jt + b * S::TPP < NB;
 }
 
+// Tile offset of row base + r STEP for a compile-time r: off() is additive where
+// STEP or (BASE8) base is a multiple of 8 rows, so that the constant part folds
+// into the access.
+template <class S, int STEP, bool BASE8 = false>
+__device__ __forceinline__ int fx_row(int base, int r) {
+    if constexpr (S::SKD == 0 || STEP % 8 == 0 || BASE8) return S::off(base) + S::off(r * STEP);
+    else return S::off(base + r * STEP);
+}
+
 // K of fx_in for a pencil of bound e2 (packed: of sums of two such values).
 template <class S>
 __host__ __device__ constexpr int fx_kin(int e2, bool packed) {
@@ -323,10 +332,9 @@ __device__ __forceinline__ FxStep fx_step(int h) {
     return s;
 }
 
-// Shared words per pencil: the largest doubled high word of its input, the
-// largest high words after the first and the second pass (all zero on entry),
-// and fx_out's eb for values left in fixed point.
-constexpr int FX_WORDS = 4;
+// Shared words per pencil: the largest doubled high word of its input, and the
+// largest high words after the first and the second pass.
+constexpr int FX_WORDS = 3;
 
 // Stage the twiddle table (cos, sin of 2 pi m / L as 2^-62 (h 2^32 + l) pairs)
 // with the sign of one direction, and clear the n pencil maxima.
@@ -340,39 +348,41 @@ __device__ __forceinline__ void fx_stage_twiddles(int4* s_tw, const int4* g_tw) 
 }
 
 // Where pencil_fx takes its input from and leaves its output.
-enum FxIn { FX_IN_GLOBAL, FX_IN_TILE, FX_IN_FIXED };     // ld(e): doubles; the tile: doubles; the tile: packed fixed point
+enum FxIn { FX_IN_GLOBAL, FX_IN_TILE };                  // ld(e); the tile
 enum FxOut { FX_OUT_GLOBAL, FX_OUT_TILE, FX_OUT_FIXED }; // st(e, value); the tile: doubles; the tile: fixed point
+
+// Scaling, twiddles and DFTs of a later pass.
+template <int R, int NS, int STEP, bool INV, int TPP, int BPT>
+__device__ __forceinline__ void fx_twiddles(C<fx> (&v)[BPT][R], const int4* tw, int jt, FxStep st) {
+    const fx half = (fx)(1ull << 31) << st.n;
+#pragma unroll
+    for (int b = 0; b < BPT; b++) {
+        const int k = (jt + TPP * b) & (NS - 1);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            v[b][r] = mk<fx>(fx_shl(v[b][r].x, st.l), fx_shl(v[b][r].y, st.l));
+            if (r > 0) v[b][r] = fx_twiddle(v[b][r], tw[(r * k) * STEP], st.n, half);
+            else v[b][r] = mk<fx>(fx_shr(v[b][r].x + (2 << st.n), st.n + 2), fx_shr(v[b][r].y + (2 << st.n), st.n + 2));
+        }
+        fx_dft<R, INV>(v[b]);
+    }
+}
 
 // One later pass of radix R after NS: read, (barrier), scale, twiddle and DFT;
 // the results stay in v.  Adds the net division to eb.
 template <class S, int R, int NS, bool INV, bool SYNC>
 __device__ __forceinline__ void fx_later_pass(C<fx> (&v)[fx_bpt<S, R>()][R], const C<fx>* tile, const int4* tw, int p,
-                                              int jt, const int* hmax, int& eb, bool active) {
+                                              int jt, const int* hmax, int& eb) {
     constexpr int NB = S::L / R, BPT = fx_bpt<S, R>(), STEP = S::L / (NS * R);
-    if (active) {
 #pragma unroll
-        for (int b = 0; b < BPT; b++)
+    for (int b = 0; b < BPT; b++)
 #pragma unroll
-            for (int r = 0; r < R; r++)
-                v[b][r] = fx_has<S, R>(b, jt) ? tile[S::off(jt + S::TPP * b + r * NB) + p] : mk<fx>(0, 0);
-    }
+        for (int r = 0; r < R; r++)
+            v[b][r] = fx_has<S, R>(b, jt) ? tile[fx_row<S, NB>(jt + S::TPP * b, r) + p] : mk<fx>(0, 0);
     const FxStep st = fx_step<R>(hmax[p]);
     if (SYNC) __syncthreads();
     eb += st.d;
-    if (active) {
-        const fx half = (fx)(1ull << 31) << st.n;
-#pragma unroll
-        for (int b = 0; b < BPT; b++) {
-            const int k = (jt + S::TPP * b) & (NS - 1);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                v[b][r] = mk<fx>(fx_shl(v[b][r].x, st.l), fx_shl(v[b][r].y, st.l));
-                if (r > 0) v[b][r] = fx_twiddle(v[b][r], tw[(r * k) * STEP], st.n, half);
-                else v[b][r] = mk<fx>(fx_shr(v[b][r].x + (2 << st.n), st.n + 2), fx_shr(v[b][r].y + (2 << st.n), st.n + 2));
-            }
-            fx_dft<R, INV>(v[b]);
-        }
-    }
+    fx_twiddles<R, NS, STEP, INV, S::TPP, BPT>(v, tw, jt, st);
 }
 
 // Index of output r of butterfly j of a pass of radix R after NS.
@@ -393,7 +403,7 @@ __device__ __forceinline__ void fx_write(C<fx>* tile, const C<fx> (&v)[fx_bpt<S,
 #pragma unroll
         for (int r = 0; r < R; r++)
             if (!((zout >> r) & 1u)) {
-                tile[S::off(d + r * NS) + p] = v[b][r];
+                tile[fx_row<S, NS, NS == 1 && R % 8 == 0>(d, r) + p] = v[b][r];
                 const int x = (int)(v[b][r].x >> 32), y = (int)(v[b][r].y >> 32);
                 hi = max(hi, max(x, y));
                 lo = min(lo, min(x, y));
@@ -423,7 +433,7 @@ __device__ __forceinline__ void fx_finish(C<double>* tile, const C<fx> (&v)[fx_b
             const int d = fx_dest<R, NS>(jt + S::TPP * b);
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                if constexpr (OUT == FX_OUT_TILE) { if (!((ZOUT >> r) & 1u)) tile[S::off(d + r * NS) + p] = o[b][r]; }
+                if constexpr (OUT == FX_OUT_TILE) { if (!((ZOUT >> r) & 1u)) tile[fx_row<S, NS, NS == 1 && R % 8 == 0>(d, r) + p] = o[b][r]; }
                 else st(d + r * NS, o[b][r]);
             }
         }
@@ -431,190 +441,286 @@ __device__ __forceinline__ void fx_finish(C<double>* tile, const C<fx> (&v)[fx_b
 }
 
 // Transform S::P pencils (thread: pencil p, butterflies jt + b TPP).  smax:
-// FX_WORDS arrays of P shared words, zero on entry but for the first one with
-// FX_IN_FIXED (the pencils' largest doubled high words).  The caller synchronises before, except
-// that FX_IN_GLOBAL does so itself once its loads are issued (staged twiddles
-// and cleared maxima become visible there); FX_OUT_TILE / FX_OUT_FIXED return
-// synchronised.  PRUNE as in pencil_fft_s: inputs of the removed band are
-// taken as zero, outputs in it are not computed (st gets zeros).
-// Threads with active = false only take part in the barriers.
+// FX_WORDS arrays of P shared words, zero on entry.  The caller synchronises
+// before, except that FX_IN_GLOBAL does so itself once its loads are issued
+// (staged twiddles and cleared maxima become visible there); FX_OUT_TILE returns
+// synchronised.  PRUNE as in pencil_fft_s: inputs of the removed band are taken
+// as zero, outputs in it are not computed (st gets zeros).
 template <class S, bool INV, bool PRUNE, FxIn IN, FxOut OUT, class Ld, class St>
-__device__ __forceinline__ void pencil_fx(C<double>* tile, const int4* tw, unsigned* smax, Ld ld, St st, bool active = true) {
+__device__ __forceinline__ void pencil_fx(C<double>* tile, const int4* tw, unsigned* smax, Ld ld, St st) {
     constexpr int L = S::L, R1 = S::R1, NB1 = L / R1, BPT1 = fx_bpt<S, R1>();
     constexpr int NPASS = S::R3 > 1 ? 3 : S::R2 > 1 ? 2 : 1;
     constexpr int RL = NPASS == 3 ? S::R3 : S::R2;
     constexpr unsigned ZI = (PRUNE && INV && NPASS > 1) ? band_mask<L, R1>() : 0u;
     constexpr unsigned ZO = (PRUNE && !INV && NPASS > 1) ? band_mask<L, RL>() : 0u;
-    const int p = active ? threadIdx.x % S::P : 0, jt = active ? threadIdx.x / S::P : 0;
+    const int p = threadIdx.x % S::P, jt = threadIdx.x / S::P;
     C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
     C<fx> v[BPT1][R1];
     FxScale sc;
-    if constexpr (IN == FX_IN_FIXED) {
-        if (active) {
-#pragma unroll
-            for (int b = 0; b < BPT1; b++)
-#pragma unroll
-                for (int r = 0; r < R1; r++)
-                    v[b][r] = ((ZI >> r) & 1u) || !fx_has<S, R1>(b, jt) ? mk<fx>(0, 0)
-                                                                        : ft[S::off(jt + S::TPP * b + r * NB1) + p];
-        }
-        sc = fx_scale(smax[p] >> 1);
-        __syncthreads();
-    } else {
+    {
         C<double> d[BPT1][R1];
-        if (active) {
 #pragma unroll
-            for (int b = 0; b < BPT1; b++)
+        for (int b = 0; b < BPT1; b++)
 #pragma unroll
-                for (int r = 0; r < R1; r++) {
-                    const int e = jt + S::TPP * b + r * NB1;
-                    if (((ZI >> r) & 1u) || !fx_has<S, R1>(b, jt)) d[b][r] = mk<double>(0., 0.);
-                    else if constexpr (IN == FX_IN_GLOBAL) d[b][r] = ld(e);
-                    else d[b][r] = tile[S::off(e) + p];
-                }
-        }
+            for (int r = 0; r < R1; r++) {
+                if (((ZI >> r) & 1u) || !fx_has<S, R1>(b, jt)) d[b][r] = mk<double>(0., 0.);
+                else if constexpr (IN == FX_IN_GLOBAL) d[b][r] = ld(jt + S::TPP * b + r * NB1);
+                else d[b][r] = tile[fx_row<S, NB1>(jt + S::TPP * b, r) + p];
+            }
         if (IN == FX_IN_GLOBAL) __syncthreads();
-        if (active) {
-            unsigned h = 0;
+        unsigned h = 0;
 #pragma unroll
-            for (int b = 0; b < BPT1; b++)
+        for (int b = 0; b < BPT1; b++)
 #pragma unroll
-                for (int r = 0; r < R1; r++)
-                    if (!((ZI >> r) & 1u)) h = fx_max(h, d[b][r]);
-            atomicMax(smax + p, h);
-        }
+            for (int r = 0; r < R1; r++)
+                if (!((ZI >> r) & 1u)) h = fx_max(h, d[b][r]);
+        atomicMax(smax + p, h);
         __syncthreads();
         sc = fx_scale(smax[p] >> 1);
-        if (active) {
-            if (sc.rare) fx_scale_all<BPT1 * R1>(&d[0][0], fx_pre(sc.rare));
-            const int K = fx_kin<S>(sc.e2, false);
+        if (sc.rare) fx_scale_all<BPT1 * R1>(&d[0][0], fx_pre(sc.rare));
+        const int K = fx_kin<S>(sc.e2, false);
 #pragma unroll
-            for (int b = 0; b < BPT1; b++)
+        for (int b = 0; b < BPT1; b++)
 #pragma unroll
-                for (int r = 0; r < R1; r++) {
-                    if ((ZI >> r) & 1u) { v[b][r] = mk<fx>(0, 0); continue; }
-                    v[b][r] = fx_in(d[b][r], K);
-                }
-        }
+            for (int r = 0; r < R1; r++) v[b][r] = ((ZI >> r) & 1u) ? mk<fx>(0, 0) : fx_in(d[b][r], K);
     }
-    if (active) {
 #pragma unroll
-        for (int b = 0; b < BPT1; b++) fx_dft<R1, INV>(v[b]);
-    }
-    int eb = fx_kin<S>(sc.e2, IN == FX_IN_FIXED);
+    for (int b = 0; b < BPT1; b++) fx_dft<R1, INV>(v[b]);
+    int eb = fx_kin<S>(sc.e2, false);
     int* hm = reinterpret_cast<int*>(smax + S::P);
     constexpr bool TO_TILE = OUT != FX_OUT_GLOBAL;
     if constexpr (NPASS == 1) {
-        if (active) fx_finish<S, R1, 1, OUT, 0u>(tile, v, p, jt, sc, eb, st);
+        fx_finish<S, R1, 1, OUT, 0u>(tile, v, p, jt, sc, eb, st);
     } else {
-        if (active) fx_write<S, R1, 1>(ft, v, p, jt, 0u, hm);
+        fx_write<S, R1, 1>(ft, v, p, jt, 0u, hm);
         __syncthreads();
         constexpr bool LAST2 = NPASS == 2;
         C<fx> v2[fx_bpt<S, S::R2>()][S::R2];
-        fx_later_pass<S, S::R2, R1, INV, !LAST2 || TO_TILE>(v2, ft, tw, p, jt, hm, eb, active);
+        fx_later_pass<S, S::R2, R1, INV, !LAST2 || TO_TILE>(v2, ft, tw, p, jt, hm, eb);
         if constexpr (LAST2) {
-            if (active) fx_finish<S, S::R2, R1, OUT, ZO>(tile, v2, p, jt, sc, eb, st);
+            fx_finish<S, S::R2, R1, OUT, ZO>(tile, v2, p, jt, sc, eb, st);
         } else {
-            if (active) fx_write<S, S::R2, R1>(ft, v2, p, jt, 0u, hm + S::P);
+            fx_write<S, S::R2, R1>(ft, v2, p, jt, 0u, hm + S::P);
             __syncthreads();
             C<fx> v3[fx_bpt<S, S::R3>()][S::R3];
-            fx_later_pass<S, S::R3, R1 * S::R2, INV, TO_TILE>(v3, ft, tw, p, jt, hm + S::P, eb, active);
-            if (active) fx_finish<S, S::R3, R1 * S::R2, OUT, ZO>(tile, v3, p, jt, sc, eb, st);
+            fx_later_pass<S, S::R3, R1 * S::R2, INV, TO_TILE>(v3, ft, tw, p, jt, hm + S::P, eb);
+            fx_finish<S, S::R3, R1 * S::R2, OUT, ZO>(tile, v3, p, jt, sc, eb, st);
         }
     }
-    if (OUT == FX_OUT_FIXED && active && jt == 0) hm[2 * S::P + p] = eb;
     if (TO_TILE) __syncthreads();
 }
 
-// --------------------------------------------------- real rows in pairs
-// Two half spectra A, B (kx < Kx) per pencil into the packed sequence
-// Z = A + iB of a c2r transform, in fixed point: each mode is loaded and
-// converted once for both of its places in Z.  get(pj, k, A, B) loads; the
-// imaginary parts at kx = 0 are dropped, as a c2r transform does.
-template <class S, int NP, int NT, class Get>
-__device__ __forceinline__ void fx_fill_packed(C<double>* tile, unsigned* smax, int Kx, Get get) {
-    constexpr int L = S::L, H = L / 2, N = H * NP, NPT = (N + NT - 1) / NT;
-    constexpr bool WARP = H % 32 == 0 && NT % 32 == 0;       // a warp's entries lie in one pencil
-    C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
-    C<double> A[NPT], B[NPT];
-#pragma unroll
-    for (int i = 0; i < NPT; i++) {
-        const int idx = threadIdx.x + i * NT, k = idx % H, pj = idx / H;
-        A[i] = B[i] = mk<double>(0., 0.);
-        if ((N % NT == 0 || idx < N) && k < Kx) get(pj, k, A[i], B[i]);
-        if (k == 0) { A[i].y = 0.; B[i].y = 0.; }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NPT; i++) {
-        const int idx = threadIdx.x + i * NT, pj = idx / H;
-        unsigned h = fx_max(fx_max(0u, A[i]), B[i]);
-        if constexpr (WARP) {
-            h = __reduce_max_sync(0xffffffffu, h);
-            if ((threadIdx.x & 31) == 0 && idx < N) atomicMax(smax + pj, h);
-        } else if (N % NT == 0 || idx < N) {
-            atomicMax(smax + pj, h);
-        }
-    }
-    __syncthreads();
-    FxScale sc[NPT];
-    int rare = 0;
-#pragma unroll
-    for (int i = 0; i < NPT; i++) {
-        const int idx = threadIdx.x + i * NT;
-        sc[i] = fx_scale(N % NT == 0 || idx < N ? smax[idx / H] >> 1 : 0u);
-        rare |= sc[i].rare;
-    }
-    if (rare) {
-#pragma unroll
-        for (int i = 0; i < NPT; i++) {
-            const double pre = fx_pre(sc[i].rare);
-            A[i].x *= pre; A[i].y *= pre; B[i].x *= pre; B[i].y *= pre;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NPT; i++) {
-        const int idx = threadIdx.x + i * NT, k = idx % H, pj = idx / H;
-        if (N % NT != 0 && idx >= N) continue;
-        const int K = fx_kin<S>(sc[i].e2, true);
-        const C<fx> a = fx_in(A[i], K), b = fx_in(B[i], K);
-        ft[S::off(k) + pj] = mk<fx>(a.x - b.y, a.y + b.x);
-        ft[S::off(k == 0 ? H : L - k) + pj] = k == 0 ? mk<fx>(0, 0) : mk<fx>(a.x + b.y, b.x - a.y);
-    }
+// --------------------------------------------------- rows: one thread group per pencil
+// The x passes' pencils are contiguous in memory, so a pencil can belong to one
+// group of TPP threads (a warp at 256 points, part of one or two warps elsewhere)
+// that loads, packs, transforms and stores it with no block barrier: consecutive
+// threads of a group take consecutive rows of the tile.  Tile rows have an odd
+// stride and a skew of one entry every 8 rows, which keeps row sequences of step 1
+// and 8 free of bank conflicts.  (With the pencils spread over all warps, as in
+// the y and z passes, the 256-point hydro pass waited at 12 block barriers: 3.6 of
+// 12.5 stalled warps per issue, 783 us per launch of a 256^3 step.)
+template <int L> struct FxRowTPP { static constexpr int v = L == 192 ? 32 : L == 96 ? 16 : FxCfg<L>::TPP; };
+template <int L, bool INV, int P, class CC = FxCfg<L>>
+using FxR = Sched<L, P, P * FxRowTPP<L>::v, INV ? CC::R[0] : CC::RF[0], INV ? CC::R[1] : CC::RF[1],
+                  INV ? CC::R[2] : CC::RF[2], (P | 1), 1>;
+
+// Shared words of a block of P groups of two warps (three reductions).
+template <class S>
+constexpr int fx_group_words() { return S::TPP > 32 ? 6 * S::P : 0; }
+
+template <int TPP>
+__device__ __forceinline__ unsigned fx_group_mask() {
+    if constexpr (TPP >= 32) return 0xffffffffu;
+    else return ((1u << TPP) - 1u) << (threadIdx.x & 31 & ~(TPP - 1));
 }
 
-// The half spectra of the real rows in a tile of packed forward transforms
-// (FX_OUT_FIXED): row t is the real (t even) or imaginary part of pencil t / 2.
-// Groups of threads take the nu rows row(u) >= 0 in turn, consecutive threads
-// consecutive kx < Kx, and put(u, k, value) the spectrum times 2^sexp smul.
-template <class S, int NT, class Row, class Put>
-__device__ __forceinline__ void fx_unpack(const C<double>* tile, const unsigned* smax, int Kx, int nu, int sexp, double smul,
-                                          Row row, Put put) {
-    constexpr int G = NT % 32 == 0 ? 32 : 16;
-    static_assert(NT % G == 0, "threads come in groups");
-    const C<fx>* ft = reinterpret_cast<const C<fx>*>(tile);
-    for (int u = threadIdx.x / G; u < nu; u += NT / G) {
-        const int t = row(u);
-        if (t < 0) continue;
-        const int p = t >> 1;
-        const bool odd = t & 1;
-        const FxScale sc = fx_scale(smax[p] >> 1);
-        const int eb = (int)smax[3 * S::P + p] - 1 + sexp;
-        const auto value = [&](int k) {
-            const C<fx> z = ft[S::off(k) + p], w = ft[S::off(k == 0 ? 0 : S::L - k) + p];
-            // A = (z + conj w) / 2, B = (z - conj w) / 2i
-            const fx re = odd ? z.y + w.y : z.x + w.x, im = odd ? w.x - z.x : z.y - w.y;
-            return fx_out(mk<fx>(re, im), eb);
-        };
-        if (smul == 1.0 && !sc.rare) {
-            for (int k = threadIdx.x % G; k < Kx; k += G) put(u, k, value(k));
-        } else {
-            const double post = sc.rare ? fx_post(sc.rare) : 1.0;
-            for (int k = threadIdx.x % G; k < Kx; k += G) {
-                const C<double> o = value(k);
-                put(u, k, mk<double>((o.x * smul) * post, (o.y * smul) * post));
-            }
+template <int TPP>
+__device__ __forceinline__ void fx_group_sync(int g) {
+    static_assert(TPP == 64 || (TPP <= 32 && 32 % TPP == 0), "groups of part of a warp or of two warps");
+    if constexpr (TPP == 64) asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+    else __syncwarp(fx_group_mask<TPP>());
+}
+
+// Largest v of the group, for every thread of it; red: two shared words of this
+// use alone (groups of two warps).
+template <int TPP>
+__device__ __forceinline__ unsigned fx_group_max(unsigned v, int g, unsigned* red) {
+    if constexpr (TPP >= 32) {
+        v = __reduce_max_sync(0xffffffffu, v);
+    } else {
+#pragma unroll
+        for (int o = TPP / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(fx_group_mask<TPP>(), v, o));
+    }
+    if constexpr (TPP == 64) {
+        if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) & 1] = v;
+        fx_group_sync<64>(g);
+        v = max(red[0], red[1]);
+    }
+    return v;
+}
+
+// Write the results of a pass and return the group's largest high word (or its
+// complement); the group synchronises.
+template <class S, int R, int NS>
+__device__ __forceinline__ int fx_group_write(C<fx>* tile, const C<fx> (&v)[fx_bpt<S, R>()][R], int p, int jt, unsigned* red) {
+    int hi = 0, lo = 0;
+#pragma unroll
+    for (int b = 0; b < fx_bpt<S, R>(); b++) {
+        if (!fx_has<S, R>(b, jt)) continue;
+        const int d = fx_dest<R, NS>(jt + S::TPP * b);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            tile[fx_row<S, NS, NS == 1 && R % 8 == 0>(d, r) + p] = v[b][r];
+            const int x = (int)(v[b][r].x >> 32), y = (int)(v[b][r].y >> 32);
+            hi = max(hi, max(x, y));
+            lo = min(lo, min(x, y));
         }
+    }
+    const int h = (int)fx_group_max<S::TPP>((unsigned)max(hi, ~lo), p, red);
+    fx_group_sync<S::TPP>(p);
+    return h;
+}
+
+// Radix-R pass after NS of the group's pencil: read, synchronise, scale, twiddle, DFT.
+template <class S, int R, int NS, bool INV>
+__device__ __forceinline__ void fx_group_pass(C<fx> (&v)[fx_bpt<S, R>()][R], const C<fx>* tile, const int4* tw, int p, int jt,
+                                              int hmax, int& eb) {
+    constexpr int NB = S::L / R, BPT = fx_bpt<S, R>(), STEP = S::L / (NS * R);
+#pragma unroll
+    for (int b = 0; b < BPT; b++)
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            v[b][r] = fx_has<S, R>(b, jt) ? tile[fx_row<S, NB>(jt + S::TPP * b, r) + p] : mk<fx>(0, 0);
+    const FxStep st = fx_step<R>(hmax);
+    fx_group_sync<S::TPP>(p);
+    eb += st.d;
+    fx_twiddles<R, NS, STEP, INV, S::TPP, BPT>(v, tw, jt, st);
+}
+
+// The later passes of the group's pencil from the results v of the first one.
+// FIXED: the tile ends up with the fixed-point transform, otherwise with doubles;
+// outputs in the band of ZOUT are left out.  Synchronised on return.
+template <class S, bool INV, bool FIXED, bool PRUNE>
+__device__ __forceinline__ void fx_group_later(C<double>* tile, C<fx> (&v)[fx_bpt<S, S::R1>()][S::R1], const int4* tw, int p,
+                                               int jt, FxScale sc, int& eb, unsigned* red) {
+    constexpr int R1 = S::R1, NPASS = S::R3 > 1 ? 3 : S::R2 > 1 ? 2 : 1;
+    constexpr int RL = NPASS == 3 ? S::R3 : S::R2;
+    constexpr unsigned ZO = (PRUNE && !INV && NPASS > 1) ? band_mask<S::L, RL>() : 0u;
+    constexpr FxOut OUT = FIXED ? FX_OUT_FIXED : FX_OUT_TILE;
+    C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
+    const auto none = [](int, C<double>) {};
+#pragma unroll
+    for (int b = 0; b < fx_bpt<S, R1>(); b++) fx_dft<R1, INV>(v[b]);
+    if constexpr (NPASS == 1) {
+        fx_finish<S, R1, 1, OUT, 0u>(tile, v, p, jt, sc, eb, none);
+    } else {
+        int h = fx_group_write<S, R1, 1>(ft, v, p, jt, red + 2);
+        C<fx> v2[fx_bpt<S, S::R2>()][S::R2];
+        fx_group_pass<S, S::R2, R1, INV>(v2, ft, tw, p, jt, h, eb);
+        if constexpr (NPASS == 2) {
+            fx_finish<S, S::R2, R1, OUT, ZO>(tile, v2, p, jt, sc, eb, none);
+        } else {
+            h = fx_group_write<S, S::R2, R1>(ft, v2, p, jt, red + 4);
+            C<fx> v3[fx_bpt<S, S::R3>()][S::R3];
+            fx_group_pass<S, S::R3, R1 * S::R2, INV>(v3, ft, tw, p, jt, h, eb);
+            fx_finish<S, S::R3, R1 * S::R2, OUT, ZO>(tile, v3, p, jt, sc, eb, none);
+        }
+    }
+    fx_group_sync<S::TPP>(p);
+}
+
+// c2r: two half spectra A, B (kx < Kx) into the packed sequence Z = A + iB in
+// fixed point (each mode is loaded and converted once for both of its places in
+// Z), then the inverse transform, whose real and imaginary parts are the two rows
+// (doubles in the tile).  get(k, A, B) loads; the imaginary parts at kx = 0 are
+// dropped, as a c2r transform does.
+template <class S, bool PRUNE, class Get>
+__device__ __forceinline__ void fx_group_c2r(C<double>* tile, const int4* tw, int p, int jt, int Kx, unsigned* red, Get get) {
+    constexpr int L = S::L, H = L / 2, TPP = S::TPP, NPT = (H + TPP - 1) / TPP, R1 = S::R1, NB1 = L / R1;
+    constexpr unsigned ZI = (PRUNE && S::R2 > 1) ? band_mask<L, R1>() : 0u;
+    C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
+    FxScale sc;
+    {
+        C<double> AB[NPT][2];
+        unsigned h = 0;
+#pragma unroll
+        for (int i = 0; i < NPT; i++) {
+            const int k = jt + TPP * i;
+            AB[i][0] = AB[i][1] = mk<double>(0., 0.);
+            if (k < Kx) get(k, AB[i][0], AB[i][1]);
+            if (k == 0) { AB[i][0].y = 0.; AB[i][1].y = 0.; }
+        }
+#pragma unroll
+        for (int i = 0; i < NPT; i++) h = fx_max(fx_max(h, AB[i][0]), AB[i][1]);
+        sc = fx_scale(fx_group_max<TPP>(h, p, red) >> 1);
+        if (sc.rare) fx_scale_all<2 * NPT>(&AB[0][0], fx_pre(sc.rare));
+        const int K = fx_kin<S>(sc.e2, true);
+#pragma unroll
+        for (int i = 0; i < NPT; i++) {
+            const int k = jt + TPP * i;
+            if (H % TPP != 0 && k >= H) continue;
+            const C<fx> a = fx_in(AB[i][0], K), b = fx_in(AB[i][1], K);
+            ft[S::off(k) + p] = mk<fx>(a.x - b.y, a.y + b.x);
+            ft[S::off(k == 0 ? H : L - k) + p] = k == 0 ? mk<fx>(0, 0) : mk<fx>(a.x + b.y, b.x - a.y);
+        }
+    }
+    fx_group_sync<TPP>(p);
+    C<fx> v[fx_bpt<S, R1>()][R1];
+#pragma unroll
+    for (int b = 0; b < fx_bpt<S, R1>(); b++)
+#pragma unroll
+        for (int r = 0; r < R1; r++)
+            v[b][r] = ((ZI >> r) & 1u) || !fx_has<S, R1>(b, jt) ? mk<fx>(0, 0) : ft[fx_row<S, NB1>(jt + TPP * b, r) + p];
+    fx_group_sync<TPP>(p);
+    int eb = fx_kin<S>(sc.e2, true);
+    fx_group_later<S, true, false, PRUNE>(tile, v, tw, p, jt, sc, eb, red);
+}
+
+// r2c: the forward transform of the packed rows ld(e) (real and imaginary part),
+// then their half spectra times 2^sexp smul: put0(k, value), put1(k, value) for
+// kx < Kx.
+template <class S, bool PRUNE, class Ld, class Put0, class Put1>
+__device__ __forceinline__ void fx_group_r2c(C<double>* tile, const int4* tw, int p, int jt, int Kx, int sexp, double smul,
+                                             unsigned* red, Ld ld, Put0 put0, Put1 put1) {
+    constexpr int L = S::L, TPP = S::TPP, R1 = S::R1, NB1 = L / R1, BPT = fx_bpt<S, R1>();
+    FxScale sc;
+    C<fx> v[BPT][R1];
+    {
+        C<double> d[BPT][R1];
+        unsigned h = 0;
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R1; r++) d[b][r] = fx_has<S, R1>(b, jt) ? ld(jt + TPP * b + r * NB1) : mk<double>(0., 0.);
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R1; r++) h = fx_max(h, d[b][r]);
+        sc = fx_scale(fx_group_max<TPP>(h, p, red) >> 1);
+        if (sc.rare) fx_scale_all<BPT * R1>(&d[0][0], fx_pre(sc.rare));
+        const int K = fx_kin<S>(sc.e2, false);
+#pragma unroll
+        for (int b = 0; b < BPT; b++)
+#pragma unroll
+            for (int r = 0; r < R1; r++) v[b][r] = fx_in(d[b][r], K);
+    }
+    fx_group_sync<TPP>(p);                 // ld may read the tile
+    int eb = fx_kin<S>(sc.e2, false);
+    fx_group_later<S, false, true, PRUNE>(tile, v, tw, p, jt, sc, eb, red);
+    const C<fx>* ft = reinterpret_cast<const C<fx>*>(tile);
+    eb += sexp - 1;
+    const bool plain = smul == 1.0 && !sc.rare;
+    const double post = sc.rare ? fx_post(sc.rare) : 1.0;
+    for (int k = jt; k < Kx; k += TPP) {
+        const C<fx> z = ft[S::off(k) + p], w = ft[S::off(k == 0 ? 0 : L - k) + p];
+        // A = (z + conj w) / 2, B = (z - conj w) / 2i
+        C<double> o[2] = {fx_out(mk<fx>(z.x + w.x, z.y - w.y), eb), fx_out(mk<fx>(z.y + w.y, w.x - z.x), eb)};
+        if (!plain) {
+            fx_scale_all<2>(o, smul);
+            fx_scale_all<2>(o, post);
+        }
+        put0(k, o[0]);
+        put1(k, o[1]);
     }
 }
 

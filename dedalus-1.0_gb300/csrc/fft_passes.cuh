@@ -103,40 +103,46 @@ struct HasPut<Op, std::void_t<decltype(&Op::put)>> : std::true_type {};
 // Shared memory: the tile, the staged twiddles and (FP64) the pencils' scaling words.
 template <typename T, class S>
 constexpr size_t pass_smem() {
-    return S::template smem_bytes<T>() + (std::is_same<T, double>::value ? sizeof(unsigned) * FX_WORDS * S::P : 0);
+    constexpr int words = S::SKD ? fx_group_words<S>() : FX_WORDS * S::P;
+    return S::template smem_bytes<T>() + (std::is_same<T, double>::value ? sizeof(unsigned) * words : 0);
 }
 
 // FP64: fixed-point transforms (fft_fixed.cuh).
 template <class S, bool INV, bool LD_E, bool ST_E, bool PRUNE, class Op>
-__device__ __forceinline__ void fx_pass_body(const Op& op, C<double>* tile, const int4* tw, unsigned* smax, int fld, int s,
+__device__ __forceinline__ void fx_pass_body(const Op& op, C<double>* tile, const int4* tw, unsigned* words, int fld, int s,
                                              int f0, int npen) {
     constexpr int L = S::L, P = S::P, PS = S::PS, NT = S::NT;
-    static_assert(S::SKD == 0, "plain tile rows");
-    const int f = f0 + threadIdx.x % P;
-    const auto ld = [&](int e) { return f < npen ? op.load(fld, s, e, f) : mk<double>(0., 0.); };
-    const auto st = [&](int e, C<double> c) { if constexpr (HasPut<Op>::value) { if (f < npen) op.put(fld, s, e, f, c); } };
     constexpr int RR = RealRows<Op>::kind;
-    constexpr FxIn IN = RR == 1 ? FX_IN_FIXED : LD_E ? FX_IN_TILE : FX_IN_GLOBAL;
-    constexpr FxOut OUT = RR == 2 ? FX_OUT_FIXED : ST_E ? FX_OUT_TILE : FX_OUT_GLOBAL;
-    if constexpr (RR == 1) {
-        fx_fill_packed<S, P, NT>(tile, smax, op.Kx, [&](int pj, int k, C<double>& A, C<double>& B) {
-            if (f0 + pj < npen) op.load_pair(fld, k, f0 + pj, A, B);
-        });
+    if constexpr (RR != 0) {               // one thread group per pair of rows
+        constexpr int TPP = S::TPP;
+        const int p = threadIdx.x / TPP, jt = threadIdx.x % TPP, f = f0 + p;
         __syncthreads();
-    } else if constexpr (LD_E) {
-        load_tile<double, L, P, PS, NT>(op, tile, fld, s, f0, npen);
-        __syncthreads();
-    }
-    pencil_fx<S, INV, PRUNE, IN, OUT>(tile, tw, smax, ld, st);
-    if constexpr (RR == 2) {
-        fx_unpack<S, NT>(tile, smax, op.Kx, 2 * P, op.sexp, op.smul,
-                         [&](int u) { return 2 * f0 + u < op.nrows ? u : -1; },
-                         [&](int u, int k, C<double> c) { op.put_row(fld, 2 * f0 + u, k, c); });
-    } else if constexpr (ST_E) {
-        const int nst = op.nstore();
-        for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
-            const int e = idx % nst, p = idx / nst;
-            if (f0 + p < npen) op.put(fld, s, e, f0 + p, tile[e * PS + p]);
+        if (f >= npen) return;
+        if constexpr (RR == 1) {
+            fx_group_c2r<S, PRUNE>(tile, tw, p, jt, op.Kx, words + 6 * p,
+                                   [&](int k, C<double>& A, C<double>& B) { op.load_pair(fld, k, f, A, B); });
+            for (int e = jt; e < L; e += TPP) op.put(fld, s, e, f, tile[S::off(e) + p]);
+        } else {
+            fx_group_r2c<S, PRUNE>(tile, tw, p, jt, op.Kx, op.sexp, op.smul, words + 6 * p,
+                                   [&](int e) { return op.load(fld, s, e, f); },
+                                   [&](int k, C<double> c) { op.put_row(fld, 2 * f, k, c); },
+                                   [&](int k, C<double> c) { if (2 * f + 1 < op.nrows) op.put_row(fld, 2 * f + 1, k, c); });
+        }
+    } else {
+        const int f = f0 + threadIdx.x % P;
+        const auto ld = [&](int e) { return f < npen ? op.load(fld, s, e, f) : mk<double>(0., 0.); };
+        const auto st = [&](int e, C<double> c) { if (f < npen) op.put(fld, s, e, f, c); };
+        if constexpr (LD_E) {
+            load_tile<double, L, P, PS, NT>(op, tile, fld, s, f0, npen);
+            __syncthreads();
+        }
+        pencil_fx<S, INV, PRUNE, LD_E ? FX_IN_TILE : FX_IN_GLOBAL, ST_E ? FX_OUT_TILE : FX_OUT_GLOBAL>(tile, tw, words, ld, st);
+        if constexpr (ST_E) {
+            const int nst = op.nstore();
+            for (int idx = threadIdx.x; idx < nst * P; idx += NT) {
+                const int e = idx % nst, p = idx / nst;
+                if (f0 + p < npen) op.put(fld, s, e, f0 + p, tile[e * PS + p]);
+            }
         }
     }
 }
@@ -151,18 +157,19 @@ __global__ void __launch_bounds__(S::NT, MB) k_pass(const Op op, int nfield) {
     const int s = blockIdx.y + 65535 * blockIdx.z;
     const int npen = op.npencil();
     if constexpr (std::is_same<T, double>::value) {
-        int4* tw = reinterpret_cast<int4*>(tile + L * PS);
-        unsigned* smax = reinterpret_cast<unsigned*>(tw + L);
+        int4* tw = reinterpret_cast<int4*>(tile + S::span);
+        unsigned* words = reinterpret_cast<unsigned*>(tw + L);
         fx_stage_twiddles<L, INV>(tw, op.tw);
-        for (int i = threadIdx.x; i < FX_WORDS * P; i += NT) smax[i] = 0u;
+        if constexpr (RealRows<Op>::kind == 0)
+            for (int i = threadIdx.x; i < FX_WORDS * P; i += NT) words[i] = 0u;
         grid_wait();
         if constexpr (HasKept<Op>::value) {
             if (op.kept() == kept23(L)) {
-                fx_pass_body<S, INV, LD_E, ST_E, true>(op, tile, tw, smax, fld, s, f0, npen);
+                fx_pass_body<S, INV, LD_E, ST_E, true>(op, tile, tw, words, fld, s, f0, npen);
                 return;
             }
         }
-        fx_pass_body<S, INV, LD_E, ST_E, false>(op, tile, tw, smax, fld, s, f0, npen);
+        fx_pass_body<S, INV, LD_E, ST_E, false>(op, tile, tw, words, fld, s, f0, npen);
     } else {
         C<T>* tw = tile + L * PS;
         load_twiddles<T, L>(tw, op.tw);
@@ -215,7 +222,10 @@ int launch_pass_sched(const Op& op, int npencil, int nslow, int nfield, cudaStre
 // default 32 pencils, but 11 tiles of 4.
 template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
 int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
-    if constexpr (std::is_same<T, double>::value)
+    if constexpr (std::is_same<T, double>::value && RealRows<Op>::kind != 0) {
+        constexpr int TPP = FxRowTPP<L>::v, P = TPP >= 4 ? 256 / TPP : 64;   // about 256 threads
+        return launch_pass_sched<T, FxR<L, INV, P>, INV, LD_E, ST_E, 1024 / (P * TPP)>(op, npencil, nslow, nfield, st, "");
+    } else if constexpr (std::is_same<T, double>::value)
         return launch_pass_sched<T, FxS<L, INV>, INV, LD_E, ST_E, FxCfg<L>::MB>(op, npencil, nslow, nfield, st, "");
     else   // FP32 inverse passes at 256 points: 5 blocks (48 registers) gain 4% on 4, forward ones spill
         return launch_pass_sched<T, DefSched<L>, INV, LD_E, ST_E, (std::is_same<T, float>::value && L == 256 && INV ? 5 : 0)>(

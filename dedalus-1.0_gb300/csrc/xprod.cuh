@@ -88,25 +88,27 @@ struct ProdCfgT : ProdCfg<L, NI, NO> {
     static constexpr bool per_point = false;
     static constexpr int min_blocks = std::is_same<T, df64>::value ? 5 : 1;   // __launch_bounds__
 };
-// FP64 (fixed-point transforms): the lengths' own schedules on exactly the
-// pencils that the fields fill, as many rows as about 256 threads take, and
-// registers for 1024 threads per SM.
+// FP64 (fixed-point transforms, a thread group per pencil): exactly the pencils
+// that the fields fill, as many rows as about 256 threads take, and registers for
+// 1024 threads per SM.
 template <int L, int NI, int NO>
 struct ProdCfgT<double, L, NI, NO> {
-    static constexpr int NM = NI > NO ? NI : NO, QF = (512 / (NM * FxCfg<L>::TPP)) & ~1;
+    static constexpr int NM = NI > NO ? NI : NO, QF = (512 / (NM * FxRowTPP<L>::v)) & ~1;
     static constexpr int Q = QF < 2 ? 2 : QF > 16 ? 16 : QF;
-    using SI = FxS<L, true, NI * Q / 2>;
-    using SF = FxS<L, false, NO * Q / 2>;
+    using SI = FxR<L, true, NI * Q / 2>;
+    using SF = FxR<L, false, NO * Q / 2>;
     static constexpr int NT = ((SI::NT > SF::NT ? SI::NT : SF::NT) + 31) / 32 * 32;
     static constexpr int min_blocks = NT > 512 ? 1 : 1024 / NT;
 };
-// Hydro in divergence form on 256-point rows: 822 us per launch of a 256^3 step
-// with 4 blocks of 192 threads (80 registers) against 853 us for the general
-// schedule above; 912 us with 3 blocks, 1059 us with 2.
-template <> struct ProdCfgT<double, 256, 3, 5> : ProdCfg<256, 3, 5> { static constexpr int min_blocks = 4; };
 // 2D hydro on 64- and 128-point rows: 2 rows per block as for a single FP32 run
-template <> struct ProdCfgT<double, 64, 3, 2> : ProdCfg<64, 3, 2> { static constexpr int min_blocks = 1; };
-template <> struct ProdCfgT<double, 128, 3, 2> : ProdCfg<128, 3, 2> { static constexpr int min_blocks = 1; };
+template <int L>
+struct ProdCfg2Rows {
+    static constexpr int Q = 2, NT = (3 * FxRowTPP<L>::v + 31) / 32 * 32, min_blocks = 1;
+    using SI = FxR<L, true, 3>;
+    using SF = FxR<L, false, 2>;
+};
+template <> struct ProdCfgT<double, 64, 3, 2> : ProdCfg2Rows<64> {};
+template <> struct ProdCfgT<double, 128, 3, 2> : ProdCfg2Rows<128> {};
 // FP32 hydro in divergence form on 256-point rows: 6 inverse and 10 forward
 // pencils in tiles with unpadded rows and a skew every 8 rows (P / 2 entries),
 // and the per-point product phase.  With the odd strides 7 and 11, 41% of the
@@ -372,79 +374,114 @@ k_x_prod(int nrows, int Kx, CPtrs win, Ptrs wout, int64_t in_rs, int64_t out_rs,
     }
 }
 
-// The same pass for FP64 in fixed point (fft_fixed.cuh): the half spectra are
-// packed and the product spectra unpacked in integers, the grid-point products
-// are FP64.
+// The same pass for FP64 in fixed point (fft_fixed.cuh): a thread group loads,
+// packs and transforms a pencil's two half spectra, the block forms the grid-point
+// products in FP64, and the groups transform, unpack and store theirs.
+template <int L, class Op>
+constexpr int prod_words_fx() {
+    using CC = ProdCfgT<double, L, Op::NI, Op::NO>;
+    return fx_group_words<typename CC::SI>() + fx_group_words<typename CC::SF>();
+}
 template <int L, class Op>
 constexpr size_t prod_smem_fx() {
     using CC = ProdCfgT<double, L, Op::NI, Op::NO>;
     const size_t a = (size_t)CC::SI::span, b = (size_t)CC::SF::span;
-    return 16 * ((a > b ? a : b) + 2 * L) + sizeof(unsigned) * FX_WORDS * (CC::SI::P + CC::SF::P);
+    return 16 * ((a > b ? a : b) + 2 * L) + sizeof(unsigned) * prod_words_fx<L, Op>();
 }
 
 template <int L, bool PRUNE, class Op>
 __device__ __forceinline__ void x_prod_fx_body(int nrows, int Kx, const CPtrs& win, const Ptrs& wout, int64_t ib, int64_t ob,
-                                               C<double>* tile, const int4* twi, const int4* twf, unsigned* smi, unsigned* smf,
+                                               C<double>* tile, const int4* twi, const int4* twf, unsigned* words,
                                                int sexp, double smul, const Op& op) {
     constexpr int NI = Op::NI, NO = Op::NO;
     using CC = ProdCfgT<double, L, NI, NO>;
     using SI = typename CC::SI;
     using SF = typename CC::SF;
-    constexpr int NT = CC::NT, Q = CC::Q, NPI = (NI * Q + 1) / 2;
+    constexpr int NT = CC::NT, Q = CC::Q, NPI = NI * Q / 2, NPF = NO * Q / 2, TPP = SI::TPP;
     const int row0 = blockIdx.x * Q;
     const int nr = min(Q, nrows - row0);
-    fx_fill_packed<SI, NPI, NT>(tile, smi, Kx, [&](int pj, int k, C<double>& A, C<double>& B) {
-        const int ta = 2 * pj, tb = 2 * pj + 1;
-        const int ra = ta / NI, fa = ta % NI, rb = tb / NI, fb = tb % NI;
-        if (ra < nr) A = ldc<double>((const double2*)pick_ptr<NI>(win.p, fa) + ib + (int64_t)(row0 + ra) * Kx + k);
-        if (tb < NI * Q && rb < nr) B = ldc<double>((const double2*)pick_ptr<NI>(win.p, fb) + ib + (int64_t)(row0 + rb) * Kx + k);
-    });
+    const int p = threadIdx.x / TPP, jt = threadIdx.x % TPP;
+    if (p < NPI) {
+        const int ra = (2 * p) / NI, rb = (2 * p + 1) / NI;
+        const double2* pa = (const double2*)pick_ptr<NI>(win.p, (2 * p) % NI) + ib + (int64_t)(row0 + ra) * Kx;
+        const double2* pb = (const double2*)pick_ptr<NI>(win.p, (2 * p + 1) % NI) + ib + (int64_t)(row0 + rb) * Kx;
+        fx_group_c2r<SI, PRUNE>(tile, twi, p, jt, Kx, words + 6 * p, [&](int k, C<double>& A, C<double>& B) {
+            if (ra < nr) A = ldc<double>(pa + k);
+            if (rb < nr) B = ldc<double>(pb + k);
+        });
+    }
     __syncthreads();
-    const auto none = [](int) { return mk<double>(0., 0.); };
-    const auto drop = [](int, C<double>) {};
-    pencil_fx<SI, true, PRUNE, FX_IN_FIXED, FX_OUT_TILE>(tile, twi, smi, none, drop, threadIdx.x < SI::NT);
-    constexpr int NPT = (L * Q + NT - 1) / NT;
-    double outv[NPT][NO];
+    constexpr int NPP = (L + NT - 1) / NT;
+    if constexpr (NPP * NPF <= 12) {
+        // a grid point of all rows per thread, whole tile entries in and out
+        C<double> outv[NPP][NPF];
 #pragma unroll
-    for (int i = 0; i < NPT; i++) {
-        const int idx = threadIdx.x + i * NT;
-        if (idx < L * Q) {
-            const int e = idx % L, r = idx / L;
-            double in[NI];
+        for (int i = 0; i < NPP; i++) {
+            const int e = threadIdx.x + i * NT;
+            if (L % NT != 0 && e >= L) continue;
+            double in[2 * NPI], out[2 * NPF];
 #pragma unroll
-            for (int f = 0; f < NI; f++) {
-                const int t = r * NI + f;
-                const double* c = &tile[SI::off(e) + t / 2].x;
-                in[f] = c[t & 1];
+            for (int pj = 0; pj < NPI; pj++) {
+                const C<double> c = tile[SI::off(e) + pj];
+                in[2 * pj] = c.x;
+                in[2 * pj + 1] = c.y;
             }
-            op(in, outv[i], blockIdx.y);
+#pragma unroll
+            for (int r = 0; r < Q; r++) op(in + r * NI, out + r * NO, blockIdx.y);
+#pragma unroll
+            for (int pj = 0; pj < NPF; pj++) outv[i][pj] = mk<double>(out[2 * pj], out[2 * pj + 1]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NPP; i++) {
+            const int e = threadIdx.x + i * NT;
+            if (L % NT != 0 && e >= L) continue;
+#pragma unroll
+            for (int pj = 0; pj < NPF; pj++) tile[SF::off(e) + pj] = outv[i][pj];
+        }
+    } else {
+        constexpr int NPT = (L * Q + NT - 1) / NT;
+        double outv[NPT][NO];
+#pragma unroll
+        for (int i = 0; i < NPT; i++) {
+            const int idx = threadIdx.x + i * NT;
+            if (idx < L * Q) {
+                const int e = idx % L, r = idx / L;
+                double in[NI];
+#pragma unroll
+                for (int f = 0; f < NI; f++) {
+                    const int t = r * NI + f;
+                    const double* c = &tile[SI::off(e) + t / 2].x;
+                    in[f] = c[t & 1];
+                }
+                op(in, outv[i], blockIdx.y);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NPT; i++) {
+            const int idx = threadIdx.x + i * NT;
+            if (idx < L * Q) {
+                const int e = idx % L, r = idx / L;
+#pragma unroll
+                for (int g = 0; g < NO; g++) {
+                    const int t = r * NO + g;
+                    double* c = &tile[SF::off(e) + t / 2].x;
+                    c[t & 1] = outv[i][g];
+                }
+            }
         }
     }
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NPT; i++) {
-        const int idx = threadIdx.x + i * NT;
-        if (idx < L * Q) {
-            const int e = idx % L, r = idx / L;
-#pragma unroll
-            for (int g = 0; g < NO; g++) {
-                const int t = r * NO + g;
-                double* c = &tile[SF::off(e) + t / 2].x;
-                c[t & 1] = outv[i][g];
-            }
-        }
+    if (p < NPF) {
+        const int ra = (2 * p) / NO, rb = (2 * p + 1) / NO;
+        double2* pa = (double2*)pick_ptr<NO>(wout.p, (2 * p) % NO) + ob + (int64_t)(row0 + ra) * Kx;
+        double2* pb = (double2*)pick_ptr<NO>(wout.p, (2 * p + 1) % NO) + ob + (int64_t)(row0 + rb) * Kx;
+        fx_group_r2c<SF, PRUNE>(tile, twf, p, jt, Kx, sexp, smul, words + fx_group_words<SI>() + 6 * p,
+                                [&](int e) { return tile[SF::off(e) + p]; },
+                                [&](int k, C<double> c) { if (ra < nr) stc<double>(pa + k, c); },
+                                [&](int k, C<double> c) { if (rb < nr) stc<double>(pb + k, c); });
     }
-    if constexpr ((NO * Q) & 1) {  // the last pencil's imaginary half is unused
-        for (int e = threadIdx.x; e < L; e += NT) tile[SF::off(e) + (NO * Q) / 2].y = 0.;
-    }
-    __syncthreads();
-    pencil_fx<SF, false, PRUNE, FX_IN_TILE, FX_OUT_FIXED>(tile, twf, smf, none, drop, threadIdx.x < SF::NT);
-    // field-major, so that a block's consecutive rows of a field are written together
-    fx_unpack<SF, NT>(tile, smf, Kx, NO * Q, sexp, smul,
-                      [&](int u) { return u % Q < nr ? (u % Q) * NO + u / Q : -1; },
-                      [&](int u, int k, C<double> c) {
-                          stc<double>((double2*)pick_ptr<NO>(wout.p, u / Q) + ob + (int64_t)(row0 + u % Q) * Kx + k, c);
-                      });
 }
 
 template <int L, class Op>
@@ -453,23 +490,22 @@ k_x_prod_fx(int nrows, int Kx, CPtrs win, Ptrs wout, int64_t in_rs, int64_t out_
             const Op op) {
     using CC = ProdCfgT<double, L, Op::NI, Op::NO>;
     extern __shared__ __align__(16) unsigned char dd_smem[];
-    constexpr int NT = CC::NT, Q = CC::Q;
+    constexpr int Q = CC::Q, NT = CC::NT;
     static_assert(Q >= 2 && Q % 2 == 0, "need an even number of rows per block");
-    static_assert((Op::NI * Q + 1) / 2 <= CC::SI::P && (Op::NO * Q + 1) / 2 <= CC::SF::P, "schedule too small for Q rows");
-    static_assert(CC::SI::NT <= NT && CC::SF::NT <= NT, "schedules must fit the block");
+    static_assert(Op::NI * Q / 2 == CC::SI::P && Op::NO * Q / 2 == CC::SF::P, "a thread group per pencil");
+    static_assert(CC::SI::NT <= NT && CC::SF::NT <= NT && CC::SI::TPP == CC::SF::TPP, "schedules must fit the block");
     C<double>* tile = reinterpret_cast<C<double>*>(dd_smem);
     constexpr size_t TA = (size_t)CC::SI::span, TB = (size_t)CC::SF::span;
     int4* twi = reinterpret_cast<int4*>(tile + (TA > TB ? TA : TB));
     int4* twf = twi + L;
-    unsigned* smi = reinterpret_cast<unsigned*>(twf + L);
-    unsigned* smf = smi + FX_WORDS * CC::SI::P;
+    unsigned* words = reinterpret_cast<unsigned*>(twf + L);
     fx_stage_twiddles<L, true>(twi, gtw);
     fx_stage_twiddles<L, false>(twf, gtw);
-    for (int i = threadIdx.x; i < FX_WORDS * (CC::SI::P + CC::SF::P); i += NT) smi[i] = 0u;
     grid_wait();
+    __syncthreads();
     const int64_t ib = blockIdx.y * in_rs, ob = blockIdx.y * out_rs;  // run (batch) offsets
-    if (Kx - 1 == kept23(L)) x_prod_fx_body<L, true>(nrows, Kx, win, wout, ib, ob, tile, twi, twf, smi, smf, sexp, smul, op);
-    else x_prod_fx_body<L, false>(nrows, Kx, win, wout, ib, ob, tile, twi, twf, smi, smf, sexp, smul, op);
+    if (Kx - 1 == kept23(L)) x_prod_fx_body<L, true>(nrows, Kx, win, wout, ib, ob, tile, twi, twf, words, sexp, smul, op);
+    else x_prod_fx_body<L, false>(nrows, Kx, win, wout, ib, ob, tile, twi, twf, words, sexp, smul, op);
 }
 
 template <typename T, int L, class Op>
