@@ -19,6 +19,8 @@ does (physics.py:412-413): in a shearing box the pressure solve then keeps
 dividing by the k^2 of the first RHS time.  ``laplace_k2 = 'current'`` on the
 physics object divides by the current k^2 instead.
 """
+import ctypes
+
 import numpy as np
 import torch
 
@@ -218,6 +220,38 @@ class ReferenceOrderRHS:
             _kset(deriv['u'][i])
 
     # ------------------------------------------------- right-hand sides
+    def _advect_fused(self, data):
+        """True when dd_advect_rhs3d covers this 3D right-hand side: a static
+        basis (no shear) and axis lengths of the fused passes."""
+        return (self.ndim == 3 and not self._shear and self._representation._static_k
+                and min(self.plan(data).xshape) >= 16)
+
+    def _advect_rhs(self, data, deriv, scalar):
+        """The whole right-hand side in one library call, in the reference's
+        operator order and roundings (generic operator sequence below)."""
+        self._generic_if(deriv)
+        deriv.set_time(data.time)
+        comps = [data['u'][i] for i in range(3)] + ([data['T'].components[0]] if scalar else [])
+        outs = [deriv['u'][i] for i in range(3)] + ([deriv['T'].components[0]] if scalar else [])
+        plan = self.plan(data)
+        om = params = None
+        if self._rotation:
+            Xz, Xy, Xx = (float(v) for v in self.parameters['Omega'])
+            om = (ctypes.c_double * 3)(Xx, Xy, Xz)
+        if scalar:
+            p = self.parameters
+            params = (ctypes.c_double * 4)(float(p['g']), float(p['alpha_t']), float(p['beta']),
+                                           float(self._direction_index()))
+        n = ctypes.c_size_t()
+        _lib.call("dd_advect_workspace_size", plan.handle, int(scalar), ctypes.byref(n))
+        ws = self.workspace(n.value)
+        sp, _a = _lib.ptr_array([kval(c).data_ptr() for c in comps])
+        dp, _b = _lib.ptr_array([c.kdata.data_ptr() for c in outs])
+        _lib.call("dd_advect_rhs3d", plan.handle, int(scalar), om, params, sp, dp, dptr(ws), ws.numel(),
+                  current_stream())
+        for c in outs:
+            _kset(c)
+
     def _generic_if(self, deriv):
         if self._first_rhs or not hasattr(next(iter(deriv.fields.values()))[0], 'integrating_factor'):
             self._setup_integrating_factors(deriv)
@@ -226,6 +260,8 @@ class ReferenceOrderRHS:
     def _generic_hydro(self, data, deriv, project):
         """IncompressibleHydro.RHS (physics.py:527-586); tracer and forcing are
         refused by _finalize."""
+        if project and self._advect_fused(data):
+            return self._advect_rhs(data, deriv, False)
         self._generic_if(deriv)
         self._base_rhs(data, deriv)
         mathscalar = self.aux_fields['mathscalar']
@@ -250,6 +286,8 @@ class ReferenceOrderRHS:
 
     def _generic_boussinesq(self, data, deriv):
         """BoussinesqHydro.RHS (physics.py:664-712)."""
+        if self._advect_fused(data):
+            return self._advect_rhs(data, deriv, True)
         self._generic_hydro(data, deriv, project=False)
         mathscalar = self.aux_fields['mathscalar']
         mathvector = self.aux_fields['mathvector']

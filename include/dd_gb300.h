@@ -394,6 +394,17 @@ int dd_kspace_real(int64_t n, const void* in, const double* r, double w, int mod
                    void* stream);
 int dd_xspace_fma(int64_t n, const double* a, const double* b, double w, int accumulate, double* out, void* stream);
 
+/* ---- 3D right-hand side in the reference's advective form (static basis) ----
+ * du = P[-(u.grad)u - 2 Omega x u + g alpha_t T e_dir] and, with nscalar = 1,
+ * dT = -(u.grad)T - beta u_dir (physics.py:527-599, 664-712), FP64, from the
+ * full-layout complex128 state (u_x, u_y, u_z[, T]) into deriv (all modes; those
+ * outside the kept set have the linear terms only).  omega: (x, y, z) or NULL for no
+ * rotation; params: g, alpha_t, beta, direction index (NULL when nscalar = 0).
+ * Axis lengths 16..512. */
+int dd_advect_workspace_size(const dd_plan* plan, int nscalar, size_t* bytes);
+int dd_advect_rhs3d(const dd_plan* plan, int nscalar, const double* omega, const double* params,
+                    const void* const* state, void* const* deriv, void* work, size_t work_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
