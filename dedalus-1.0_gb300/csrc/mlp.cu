@@ -35,9 +35,7 @@ __device__ __forceinline__ void load_x_tile(MlpFwdSmem& s, const bf16* X, const 
             const int64_t row = idx ? idx[sidx] : sidx;
             v = reinterpret_cast<const uint4*>(X + row * MLP_IN)[h];
         }
-        const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-        for (int j = 0; j < 8; j++) s.x[r * LDI + 8 * h + j] = e[j];
+        *reinterpret_cast<uint4*>(s.x + r * LDI + 8 * h) = v;
     }
 }
 
@@ -75,7 +73,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
     mlp_load_weights(s, wb, p);
     const int warp = threadIdx.x >> 5, r0 = 16 * warp;
     float gw2[8][4] = {}, gw1[2][4] = {}, gw3[2][4] = {};
-    float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, sse = 0.f;
+    float gb = 0.f, gb3 = 0.f, sse = 0.f;
     for (int64_t base = (int64_t)blockIdx.x * 64; base < n; base += (int64_t)gridDim.x * 64) {
         __syncthreads();
         load_x_tile(s, X, idx, base, n);
@@ -101,18 +99,20 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
         __syncwarp();
         {   // dH2 = (dY W3) * (1 - H2^2)
             uint32_t a[4];
-            mlp_load_a(a, s.dy + r0 * LDI, LDI, 1);
+            mlp_load_a<LDI, false>(a, s.dy + r0 * LDI);
 #pragma unroll
             for (int nt = 0; nt < 8; nt++) {
                 float c[4] = {0.f, 0.f, 0.f, 0.f};
                 uint32_t b[2];
-                mlp_load_b(b, s.w3 + 8 * nt, LDH, 1);
+                mlp_load_b<LDH, true>(b, s.w3 + 8 * nt);
                 mma_bf16_16816(c, a, b);
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int r = r0 + frag_row(q), col = 8 * nt + frag_col(q);
-                    const float h = __bfloat162float(s.h2[r * LDH + col]);
-                    s.dh2[r * LDH + col] = __float2bfloat16_rn(c[q] * (1.f - h * h));
+                for (int q = 0; q < 4; q += 2) {
+                    const int o = (r0 + frag_row(q)) * LDH + 8 * nt + frag_col(q);
+                    const __nv_bfloat162 hh = *reinterpret_cast<const __nv_bfloat162*>(s.h2 + o);
+                    const float h0 = __bfloat162float(hh.x), h1 = __bfloat162float(hh.y);
+                    *reinterpret_cast<uint32_t*>(s.dh2 + o) = pack2(__float2bfloat16_rn(c[q] * (1.f - h0 * h0)),
+                                                                   __float2bfloat16_rn(c[q + 1] * (1.f - h1 * h1)));
                 }
             }
         }
@@ -120,21 +120,23 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
         {   // dH1 = (dH2 W2) * (1 - H1^2)
             uint32_t a[4][4];
 #pragma unroll
-            for (int kt = 0; kt < 4; kt++) mlp_load_a(a[kt], s.dh2 + r0 * LDH + 16 * kt, LDH, 1);
+            for (int kt = 0; kt < 4; kt++) mlp_load_a<LDH, false>(a[kt], s.dh2 + r0 * LDH + 16 * kt);
 #pragma unroll
             for (int nt = 0; nt < 8; nt++) {
                 float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int kt = 0; kt < 4; kt++) {
                     uint32_t b[2];
-                    mlp_load_b(b, s.w2 + (16 * kt) * LDH + 8 * nt, LDH, 1);
+                    mlp_load_b<LDH, true>(b, s.w2 + (16 * kt) * LDH + 8 * nt);
                     mma_bf16_16816(c, a[kt], b);
                 }
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int r = r0 + frag_row(q), col = 8 * nt + frag_col(q);
-                    const float h = __bfloat162float(s.h1[r * LDH + col]);
-                    s.dh1[r * LDH + col] = __float2bfloat16_rn(c[q] * (1.f - h * h));
+                for (int q = 0; q < 4; q += 2) {
+                    const int o = (r0 + frag_row(q)) * LDH + 8 * nt + frag_col(q);
+                    const __nv_bfloat162 hh = *reinterpret_cast<const __nv_bfloat162*>(s.h1 + o);
+                    const float h0 = __bfloat162float(hh.x), h1 = __bfloat162float(hh.y);
+                    *reinterpret_cast<uint32_t*>(s.dh1 + o) = pack2(__float2bfloat16_rn(c[q] * (1.f - h0 * h0)),
+                                                                   __float2bfloat16_rn(c[q + 1] * (1.f - h1 * h1)));
                 }
             }
         }
@@ -144,11 +146,11 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
             uint32_t a[4];
-            mlp_load_a(a, s.dh2 + (16 * kt) * LDH + 16 * warp, 1, LDH);
+            mlp_load_a<LDH, true>(a, s.dh2 + (16 * kt) * LDH + 16 * warp);
 #pragma unroll
             for (int nt = 0; nt < 8; nt++) {
                 uint32_t b[2];
-                mlp_load_b(b, s.h1 + (16 * kt) * LDH + 8 * nt, LDH, 1);
+                mlp_load_b<LDH, true>(b, s.h1 + (16 * kt) * LDH + 8 * nt);
                 mma_bf16_16816(gw2[nt], a, b);
             }
         }
@@ -156,11 +158,11 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
             uint32_t a[4];
-            mlp_load_a(a, s.dh1 + (16 * kt) * LDH + 16 * warp, 1, LDH);
+            mlp_load_a<LDH, true>(a, s.dh1 + (16 * kt) * LDH + 16 * warp);
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
                 uint32_t b[2];
-                mlp_load_b(b, s.x + (16 * kt) * LDI + 8 * nt, LDI, 1);
+                mlp_load_b<LDI, true>(b, s.x + (16 * kt) * LDI + 8 * nt);
                 mma_bf16_16816(gw1[nt], a, b);
             }
         }
@@ -168,27 +170,28 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
             uint32_t a[4];
-            mlp_load_a(a, s.dy + (16 * kt) * LDI, 1, LDI);
+            mlp_load_a<LDI, true>(a, s.dy + (16 * kt) * LDI);
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 uint32_t b[2];
-                mlp_load_b(b, s.h2 + (16 * kt) * LDH + 8 * (2 * warp + j), LDH, 1);
+                mlp_load_b<LDH, true>(b, s.h2 + (16 * kt) * LDH + 8 * (2 * warp + j));
                 mma_bf16_16816(gw3[j], a, b);
             }
         }
-        if (threadIdx.x < MLP_H) {
-            float a1 = 0.f, a2 = 0.f;
-            for (int r = 0; r < 64; r++) {
-                a1 += __bfloat162float(s.dh1[r * LDH + threadIdx.x]);
-                a2 += __bfloat162float(s.dh2[r * LDH + threadIdx.x]);
-            }
-            gb1 += a1;
-            gb2 += a2;
+        {   // bias gradients: half the block sums a column of dH1 each, half one of dH2
+            const bf16* d = (threadIdx.x < MLP_H ? s.dh1 : s.dh2) + threadIdx.x % MLP_H;
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int r = 0; r < 64; r += 4)
+#pragma unroll
+                for (int j = 0; j < 4; j++) t[j] += __bfloat162float(d[(r + j) * LDH]);
+            gb += (t[0] + t[1]) + (t[2] + t[3]);
         }
-        if (threadIdx.x < MLP_OUT) {
-            float a3 = 0.f;
-            for (int r = 0; r < 64; r++) a3 += s.dyf[r * MLP_OUT + threadIdx.x];
-            gb3 += a3;
+        if (threadIdx.x < 8 * MLP_OUT) {   // 8 rows per thread
+            float t = 0.f;
+#pragma unroll
+            for (int r = 0; r < 8; r++) t += s.dyf[(8 * (threadIdx.x / MLP_OUT) + r) * MLP_OUT + threadIdx.x % MLP_OUT];
+            gb3 += t;
         }
     }
     // every gradient entry has exactly one owner: plain stores
@@ -208,11 +211,15 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
             const int o = frag_row(q);
             if (o < MLP_OUT) P[OFF_W3 + o * MLP_H + 8 * (2 * warp + j) + frag_col(q)] = gw3[j][q];
         }
-    if (threadIdx.x < MLP_H) {
-        P[OFF_B1 + threadIdx.x] = gb1;
-        P[OFF_B2 + threadIdx.x] = gb2;
+    P[(threadIdx.x < MLP_H ? OFF_B1 : OFF_B2) + threadIdx.x % MLP_H] = gb;
+    __syncthreads();
+    if (threadIdx.x < 8 * MLP_OUT) s.dyf[threadIdx.x] = gb3;
+    __syncthreads();
+    if (threadIdx.x < MLP_OUT) {
+        float t = 0.f;
+        for (int r = 0; r < 8; r++) t += s.dyf[r * MLP_OUT + threadIdx.x];
+        P[OFF_B3 + threadIdx.x] = t;
     }
-    if (threadIdx.x < MLP_OUT) P[OFF_B3 + threadIdx.x] = gb3;
     for (int o = 16; o > 0; o >>= 1) sse += __shfl_down_sync(0xffffffffu, sse, o);
     if ((threadIdx.x & 31) == 0) s.red[warp] = sse;
     __syncthreads();
@@ -223,12 +230,24 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_grad(const bf16* __restrict
     }
 }
 
-// grad[j] = sum_b part[b][j] in block order; loss[0] = sum_b part[b][NPARAM].
-__global__ void k_mlp_reduce(const float* __restrict__ part, int nblk, float* grad, float* loss) {
+// grad[j] = sum_b part[b][j], loss[0] = sum_b part[b][NPARAM], each in a fixed order:
+// RS slices of the blocks b = s, s + RS, ... and then the slices.
+constexpr int RS = 16;
+__global__ void __launch_bounds__(32 * RS) k_mlp_reduce(const float* __restrict__ part, int nblk, float* grad, float* loss) {
     grid_wait();
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= MLP_NPARAM; j += gridDim.x * blockDim.x) {
-        float t = 0.f;
-        for (int b = 0; b < nblk; b++) t += part[(int64_t)b * MLP_PSTRIDE + j];
+    __shared__ float sum[RS][33];
+    const int l = threadIdx.x & 31, sl = threadIdx.x >> 5, j = blockIdx.x * 32 + l;
+    float t = 0.f;
+    if (j <= MLP_NPARAM) {
+#pragma unroll 4
+        for (int b = sl; b < nblk; b += RS) t += part[(int64_t)b * MLP_PSTRIDE + j];
+    }
+    sum[sl][l] = t;
+    __syncthreads();
+    if (sl == 0 && j <= MLP_NPARAM) {
+        t = 0.f;
+#pragma unroll
+        for (int r = 0; r < RS; r++) t += sum[r][l];
         if (j < MLP_NPARAM) grad[j] = t;
         else if (loss) loss[0] = t;
     }
@@ -250,8 +269,9 @@ __global__ void k_mlp_pack(const float* p, bf16* wb) {
 
 // Adam (Kingma & Ba, 2015): m = b1 m + (1 - b1) g; v = b2 v + (1 - b2) g^2;
 // p -= lr (m / bc1) / (sqrt(v / bc2) + eps) with bc = 1 - beta^step.
+// The BF16 copy (as k_mlp_pack) is written with the update.
 __global__ void k_mlp_adam(float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
-                           float bc1, float bc2) {
+                           float bc1, float bc2, bf16* wb) {
     grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < MLP_NPARAM; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
@@ -259,7 +279,13 @@ __global__ void k_mlp_adam(float* p, const float* g, float* m, float* v, float l
         const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
         m[i] = mi;
         v[i] = vi;
-        p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+        const float pi = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+        p[i] = pi;
+        const int j = i < OFF_B1 ? BOFF_W1 + (i - OFF_W1)
+                      : i >= OFF_W2 && i < OFF_B2 ? BOFF_W2 + (i - OFF_W2)
+                      : i >= OFF_W3 && i < OFF_B3 ? BOFF_W3 + (i - OFF_W3) : -1;
+        if (j >= 0) wb[j] = __float2bfloat16_rn(pi);
+        if (i < MLP_OUT * MLP_H) wb[BOFF_W3 + MLP_OUT * MLP_H + i] = __float2bfloat16_rn(0.f);   // rows 8..15
     }
 }
 
@@ -340,7 +366,7 @@ int dd_mlp_grad(const void* X, const float* T, const int64_t* idx, int64_t n, in
           launch(k_mlp_grad, nb, MLP_THREADS, sizeof(MlpSmem), st, (const bf16*)X, T, idx, n, (const bf16*)wbf16, params,
                                                                 scale, part));
     DD_LAUNCH_CHECK();
-    DD_KT("mlp_reduce", st, launch(k_mlp_reduce, ew_blocks(MLP_NPARAM + 1, 256), 256, 0, st, part, nb, grad, loss));
+    DD_KT("mlp_reduce", st, launch(k_mlp_reduce, ew_blocks(MLP_NPARAM + 1, 32), 32 * RS, 0, st, part, nb, grad, loss));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }
@@ -351,9 +377,10 @@ int dd_mlp_adam(float* params, const float* grad, float* m, float* v, int step, 
     cudaStream_t st = (cudaStream_t)stream;
     const float bc1 = 1.f - powf(beta1, (float)step), bc2 = 1.f - powf(beta2, (float)step);
     DD_KT("mlp_adam", st,
-          launch(k_mlp_adam, ew_blocks(MLP_NPARAM, 256), 256, 0, st, params, grad, m, v, lr, beta1, beta2, eps, bc1, bc2));
+          launch(k_mlp_adam, ew_blocks(MLP_NPARAM, 256), 256, 0, st, params, grad, m, v, lr, beta1, beta2, eps, bc1, bc2,
+                 (bf16*)wbf16));
     DD_LAUNCH_CHECK();
-    return dd_mlp_pack(params, wbf16, stream);
+    return DD_OK;
 }
 
 int dd_mlp_normalize(const float* raw, int64_t n, const float* norm, void* X, float* T, void* stream) {

@@ -59,20 +59,37 @@ __device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
-// A fragment (16 x 16, row major): element (r, k) at base[r * rs + k * ks]
-__device__ __forceinline__ void mlp_load_a(uint32_t a[4], const bf16* base, int rs, int ks) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    a[0] = pack2(base[g * rs + (2 * t) * ks], base[g * rs + (2 * t + 1) * ks]);
-    a[1] = pack2(base[(g + 8) * rs + (2 * t) * ks], base[(g + 8) * rs + (2 * t + 1) * ks]);
-    a[2] = pack2(base[g * rs + (2 * t + 8) * ks], base[g * rs + (2 * t + 9) * ks]);
-    a[3] = pack2(base[(g + 8) * rs + (2 * t + 8) * ks], base[(g + 8) * rs + (2 * t + 9) * ks]);
+// Fragments by ldmatrix from shared-memory rows of stride LD elements (a multiple
+// of 8, so every row starts on 16 bytes); base on 16 bytes.  (One or two 2-byte
+// loads per element pair made the training kernel LSU-bound: about 770 loads per
+// warp and tile, now 120.)
+// A fragment (16 x 16): element (r, k) at base[r LD + k], or at base[k LD + r] (TRANS).
+template <int LD, bool TRANS>
+__device__ __forceinline__ void mlp_load_a(uint32_t a[4], const bf16* base) {
+    const int l = threadIdx.x & 31, m = l >> 3;
+    const bf16* p = TRANS ? base + ((l & 7) + (m >> 1) * 8) * LD + (m & 1) * 8
+                          : base + ((l & 7) + (m & 1) * 8) * LD + (m >> 1) * 8;
+    const uint32_t sp = (uint32_t)__cvta_generic_to_shared(p);
+    if constexpr (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(sp) : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(sp) : "memory");
 }
 
-// B fragment (16 x 8, column major): element (k, n) at base[k * ks + n * ns]
-__device__ __forceinline__ void mlp_load_b(uint32_t b[2], const bf16* base, int ks, int ns) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    b[0] = pack2(base[(2 * t) * ks + g * ns], base[(2 * t + 1) * ks + g * ns]);
-    b[1] = pack2(base[(2 * t + 8) * ks + g * ns], base[(2 * t + 9) * ks + g * ns]);
+// B fragment (16 x 8): element (k, n) at base[n LD + k], or at base[k LD + n] (TRANS).
+template <int LD, bool TRANS>
+__device__ __forceinline__ void mlp_load_b(uint32_t b[2], const bf16* base) {
+    const int l = threadIdx.x & 15;
+    const bf16* p = TRANS ? base + l * LD : base + (l & 7) * LD + (l >> 3) * 8;
+    const uint32_t sp = (uint32_t)__cvta_generic_to_shared(p);
+    if constexpr (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+                     : "=r"(b[0]), "=r"(b[1]) : "r"(sp) : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
+                     : "=r"(b[0]), "=r"(b[1]) : "r"(sp) : "memory");
 }
 
 __device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], const uint32_t b[2]) {
@@ -87,14 +104,24 @@ __device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], 
 __device__ __forceinline__ int frag_row(int q) { return ((threadIdx.x & 31) >> 2) + (q >= 2 ? 8 : 0); }
 __device__ __forceinline__ int frag_col(int q) { return 2 * (threadIdx.x & 3) + (q & 1); }
 
+// n rows of LEN contiguous BF16 values to rows of stride LD, 16 bytes at a time
+// where src allows it.
+template <int LEN, int LD>
+__device__ __forceinline__ void mlp_copy_rows(bf16* dst, const bf16* src, int n) {
+    if (((uintptr_t)src & 15) == 0) {
+        constexpr int C = LEN / 8;
+        for (int i = threadIdx.x; i < n * C; i += blockDim.x)
+            *reinterpret_cast<uint4*>(dst + (i / C) * LD + (i % C) * 8) = reinterpret_cast<const uint4*>(src)[i];
+    } else {
+        for (int i = threadIdx.x; i < n * LEN; i += blockDim.x) dst[(i / LEN) * LD + i % LEN] = src[i];
+    }
+}
+
 // BF16 weights (global, unpadded) and FP32 biases into shared memory.
 __device__ inline void mlp_load_weights(MlpFwdSmem& s, const bf16* wb, const float* p) {
-    for (int i = threadIdx.x; i < MLP_H * MLP_IN; i += blockDim.x)
-        s.w1[(i / MLP_IN) * LDI + i % MLP_IN] = wb[BOFF_W1 + i];
-    for (int i = threadIdx.x; i < MLP_H * MLP_H; i += blockDim.x)
-        s.w2[(i / MLP_H) * LDH + i % MLP_H] = wb[BOFF_W2 + i];
-    for (int i = threadIdx.x; i < 16 * MLP_H; i += blockDim.x)
-        s.w3[(i / MLP_H) * LDH + i % MLP_H] = wb[BOFF_W3 + i];
+    mlp_copy_rows<MLP_IN, LDI>(s.w1, wb + BOFF_W1, MLP_H);
+    mlp_copy_rows<MLP_H, LDH>(s.w2, wb + BOFF_W2, MLP_H);
+    mlp_copy_rows<MLP_H, LDH>(s.w3, wb + BOFF_W3, 16);
     for (int i = threadIdx.x; i < MLP_H; i += blockDim.x) {
         s.b1[i] = p[OFF_B1 + i];
         s.b2[i] = p[OFF_B2 + i];
@@ -118,17 +145,18 @@ struct MlpW {
 __device__ inline void mlp_forward16(const MlpW& W, const bf16* x, bf16* h1, bf16* h2, float y[4]) {
     {   // H1 = tanh(X W1^T + b1)
         uint32_t a[4];
-        mlp_load_a(a, x, LDI, 1);
+        mlp_load_a<LDI, false>(a, x);
 #pragma unroll
         for (int nt = 0; nt < MLP_H / 8; nt++) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t b[2];
-            mlp_load_b(b, W.w1 + (8 * nt) * LDI, 1, LDI);
+            mlp_load_b<LDI, false>(b, W.w1 + (8 * nt) * LDI);
             mma_bf16_16816(c, a, b);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
+            for (int q = 0; q < 4; q += 2) {      // two adjacent columns per store
                 const int col = 8 * nt + frag_col(q);
-                h1[frag_row(q) * LDH + col] = __float2bfloat16_rn(tanhf(c[q] + W.b1[col]));
+                *reinterpret_cast<uint32_t*>(h1 + frag_row(q) * LDH + col) =
+                    pack2(__float2bfloat16_rn(tanhf(c[q] + W.b1[col])), __float2bfloat16_rn(tanhf(c[q + 1] + W.b1[col + 1])));
             }
         }
     }
@@ -136,20 +164,21 @@ __device__ inline void mlp_forward16(const MlpW& W, const bf16* x, bf16* h1, bf1
     {   // H2 = tanh(H1 W2^T + b2)
         uint32_t a[4][4];
 #pragma unroll
-        for (int kt = 0; kt < 4; kt++) mlp_load_a(a[kt], h1 + 16 * kt, LDH, 1);
+        for (int kt = 0; kt < 4; kt++) mlp_load_a<LDH, false>(a[kt], h1 + 16 * kt);
 #pragma unroll
         for (int nt = 0; nt < MLP_H / 8; nt++) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int kt = 0; kt < 4; kt++) {
                 uint32_t b[2];
-                mlp_load_b(b, W.w2 + (8 * nt) * LDH + 16 * kt, 1, LDH);
+                mlp_load_b<LDH, false>(b, W.w2 + (8 * nt) * LDH + 16 * kt);
                 mma_bf16_16816(c, a[kt], b);
             }
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
+            for (int q = 0; q < 4; q += 2) {      // two adjacent columns per store
                 const int col = 8 * nt + frag_col(q);
-                h2[frag_row(q) * LDH + col] = __float2bfloat16_rn(tanhf(c[q] + W.b2[col]));
+                *reinterpret_cast<uint32_t*>(h2 + frag_row(q) * LDH + col) =
+                    pack2(__float2bfloat16_rn(tanhf(c[q] + W.b2[col])), __float2bfloat16_rn(tanhf(c[q + 1] + W.b2[col + 1])));
             }
         }
     }
@@ -159,8 +188,8 @@ __device__ inline void mlp_forward16(const MlpW& W, const bf16* x, bf16* h1, bf1
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
             uint32_t a[4], b[2];
-            mlp_load_a(a, h2 + 16 * kt, LDH, 1);
-            mlp_load_b(b, W.w3 + 16 * kt, 1, LDH);
+            mlp_load_a<LDH, false>(a, h2 + 16 * kt);
+            mlp_load_b<LDH, false>(b, W.w3 + 16 * kt);
             mma_bf16_16816(c, a, b);
         }
 #pragma unroll
