@@ -100,6 +100,17 @@ int fft_c2r(const dd_plan* pl, int nf, const void* const* k, XT* const* x, void*
     return DD_OK;
 }
 
+// The x pass alone: nf fields at [z][y][kxc] to grid-point values.
+template <typename T, typename XT = double>
+int fft_x_c2r3(const dd_plan* pl, int nf, const void* const* w2, XT* const* x, cudaStream_t st) {
+    const Geo3& g = pl->g3;
+    CPtrs in{}; Ptrs xo{};
+    for (int f = 0; f < nf; f++) { in.p[f] = w2[f]; xo.p[f] = x[f]; }
+    const int nrows = g.Nz * g.Ny;
+    OpXc2r3<T, XT> c{nrows, g.Nx, g.Kx, in, xo, TwSel<T>::x(pl)};
+    return launch_pass_len<T, true, true, true>(g.Nx, c, (nrows + 1) / 2, 1, nf, st);
+}
+
 // zero_nonkept = false leaves the entries outside the kept set unwritten (for
 // internal callers that read kept modes only).
 template <typename T, typename XT = double>
@@ -150,10 +161,12 @@ int fft_r2c(const dd_plan* pl, int nf, const XT* const* x, void* const* k, void*
 }
 
 #define DD_FFT_INSTANTIATE(EXT, T)                                                                       \
+    EXT template int fft_x_c2r3<T>(const dd_plan*, int, const void* const*, double* const*, cudaStream_t);     \
     EXT template int fft_c2r<T>(const dd_plan*, int, const void* const*, double* const*, void*, size_t, cudaStream_t); \
     EXT template int fft_r2c<T>(const dd_plan*, int, const double* const*, void* const*, void*, size_t, cudaStream_t, \
                                 bool);
 #define DD_FFT_INSTANTIATE_X(EXT, T, XT)                                                                 \
+    EXT template int fft_x_c2r3<T, XT>(const dd_plan*, int, const void* const*, XT* const*, cudaStream_t);     \
     EXT template int fft_c2r<T, XT>(const dd_plan*, int, const void* const*, XT* const*, void*, size_t,        \
                                     cudaStream_t);                                                          \
     EXT template int fft_r2c<T, XT>(const dd_plan*, int, const XT* const*, void* const*, void*, size_t,        \

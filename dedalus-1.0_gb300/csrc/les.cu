@@ -34,7 +34,6 @@ __device__ __forceinline__ void les_kept(const Geo3& g, int64_t i, int& ky_i, in
 __device__ __forceinline__ double2 les_ik(double2 a, double k) { return make_double2(-(k * a.y), k * a.x); }
 
 // gk[3 a + j] = i k_j y_a on the kept modes (full layout out).
-template <bool COMPACT>
 __global__ void k_les_grad9(Geo3 g, const double* kx, const double* ky, const double* kz, CPtrs y, Ptrs gk) {
     grid_wait();
     const int64_t n = (int64_t)g.Ky * g.Kz * g.Kx;
@@ -43,10 +42,9 @@ __global__ void k_les_grad9(Geo3 g, const double* kx, const double* ky, const do
         int64_t o;
         les_kept(g, i, ky_i, kz_i, ix, o);
         const double kv[3] = {kx[ix], ky[ky_i], kz[kz_i]};
-        const int64_t src = COMPACT ? i : o;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            const double2 u = ((const double2*)y.p[a])[src];
+            const double2 u = ((const double2*)y.p[a])[o];
 #pragma unroll
             for (int j = 0; j < 3; j++) ((double2*)gk.p[3 * a + j])[o] = les_ik(u, kv[j]);
         }
@@ -415,7 +413,7 @@ static LesWork les_carve(const dd_plan* p, void* work) {
 
 // Gradients at the grid points: into w.gxf as float when xf32 (FP32
 // transforms only), else into w.gx as double.
-static int les_grads(const dd_plan* p, int prec, bool compact, const void* const* y, const LesWork& w,
+static int les_grads(const dd_plan* p, int prec, const void* const* y, const LesWork& w,
                      bool xf32, cudaStream_t st) {
     const Geo3& g = p->g3;
     CPtrs yc{};
@@ -423,8 +421,7 @@ static int les_grads(const dd_plan* p, int prec, bool compact, const void* const
     for (int a = 0; a < 3; a++) yc.p[a] = y[a];
     for (int f = 0; f < 9; f++) gk.p[f] = w.gk[f];
     const unsigned nb = les_grid((int64_t)g.Ky * g.Kz * g.Kx);
-    if (compact) DD_KT("les_grad9", st, launch(k_les_grad9<true>, nb, 256, 0, st, g, p->kx, p->ky, p->kz, yc, gk));
-    else DD_KT("les_grad9", st, launch(k_les_grad9<false>, nb, 256, 0, st, g, p->kx, p->ky, p->kz, yc, gk));
+    DD_KT("les_grad9", st, launch(k_les_grad9, nb, 256, 0, st, g, p->kx, p->ky, p->kz, yc, gk));
     DD_LAUNCH_CHECK();
     const void* kin[9];
     for (int f = 0; f < 9; f++) kin[f] = w.gk[f];
@@ -460,12 +457,25 @@ static int les_mlp(const dd_plan* p, const dd_closure* cl, const GT* const* gxi,
     return DD_OK;
 }
 
-int les_closure_add(const dd_plan* p, const LesHook& h, int prec, bool compact, const void* const* y,
-                    void* const* nc, cudaStream_t st) {
+int les_grad_bufs(const dd_plan* p, const LesHook& h, int prec, GradBufs* out) {
     DD_CHECK_ARG(h.wb >= les_work_bytes(p), "closure workspace too small");
     const LesWork w = les_carve(p, h.work);
+    const Geo3& g = p->g3;
+    const size_t e = prec == DD_FP32 ? sizeof(C<float>) : sizeof(C<double>);
+    for (int f = 0; f < 9; f++) {          // as fft_c2r lays out its workspace
+        out->w1[f] = (char*)w.fw + e * (size_t)f * g.w1count();
+        out->w2[f] = (char*)w.fw + e * ((size_t)9 * g.w1count() + (size_t)f * g.w2count());
+    }
+    return DD_OK;
+}
+
+int les_closure_add(const dd_plan* p, const LesHook& h, int prec, void* const* nc, cudaStream_t st) {
+    GradBufs gb;
+    DD_TRY(les_grad_bufs(p, h, prec, &gb));
+    const LesWork w = les_carve(p, h.work);
     const bool f32 = prec == DD_FP32;
-    DD_TRY(les_grads(p, prec, compact, y, w, f32, st));
+    if (f32) DD_TRY((fft_x_c2r3<float, float>(p, 9, gb.w2, w.gxf, st)));
+    else DD_TRY(fft_x_c2r3<double>(p, 9, gb.w2, w.gx, st));
     // the stresses overwrite gradients 0..5; k_les_add reads the kept modes
     // only, so the forward transform leaves the rest unwritten
     void* kout[6];
@@ -565,7 +575,7 @@ int dd_les_gradients(const dd_plan* p, const void* const* u, double* const* gx, 
     for (int f = 0; f < 9; f++) DD_CHECK_ARG(gx[f], "null gradient %d", f);
     cudaStream_t st = (cudaStream_t)stream;
     const LesWork w = les_carve(p, work);
-    DD_TRY(les_grads(p, precision, false, u, w, false, st));
+    DD_TRY(les_grads(p, precision, u, w, false, st));
     const int64_t xb = p->g3.xcount() * (int64_t)sizeof(double);
     for (int f = 0; f < 9; f++) DD_CUDA(cudaMemcpyAsync(gx[f], w.gx[f], xb, cudaMemcpyDeviceToDevice, st));
     return DD_OK;
@@ -595,7 +605,7 @@ int dd_les_stress(const dd_plan* p, const void* const* u, double* const* tau, co
     cudaStream_t st = (cudaStream_t)stream;
     const LesWork w = les_carve(p, work);
     const bool f32 = precision == DD_FP32;
-    DD_TRY(les_grads(p, precision, false, u, w, f32, st));
+    DD_TRY(les_grads(p, precision, u, w, f32, st));
     if (f32) return les_mlp<float, double>(p, cl, w.gxf, tau, st);
     return les_mlp<double, double>(p, cl, w.gx, tau, st);
 }

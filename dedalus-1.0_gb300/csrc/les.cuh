@@ -4,6 +4,7 @@
 #pragma once
 #include "dd_common.cuh"
 #include "plan.cuh"
+#include "rhs3d_impl.cuh"
 
 namespace dd {
 
@@ -18,9 +19,11 @@ struct LesHook {
 // grid-point values, transform workspace).
 size_t les_work_bytes(const dd_plan* p);
 
-// nc[i] += -(i k_j tau_ij)^ on the kept modes (compact complex128 layout), for
-// the state y (3 velocity components, full layout, or compact when compact).
-int les_closure_add(const dd_plan* p, const LesHook& h, int prec, bool compact, const void* const* y,
-                    void* const* nc, cudaStream_t st);
+// Buffers of the nine gradients' z and y passes in the closure's scratch region.
+int les_grad_bufs(const dd_plan* p, const LesHook& h, int prec, GradBufs* out);
+
+// nc[i] += -(i k_j tau_ij)^ on the kept modes (compact complex128 layout), from the
+// gradients that the z and y passes left in les_grad_bufs.
+int les_closure_add(const dd_plan* p, const LesHook& h, int prec, void* const* nc, cudaStream_t st);
 
 }  // namespace dd

@@ -426,11 +426,11 @@ static unsigned ew_grid(int64_t n) {
 
 template <int PH>
 static int nonlinear3_any(const dd_plan* pl, int prec, bool compact, const void* const* u, double inv_fpr,
-                          const Work3& w, cudaStream_t st) {
-    if (prec == DD_FP64) return compact ? nonlinear3<double, true, PH>(pl, u, inv_fpr, w, st)
-                                        : nonlinear3<double, false, PH>(pl, u, inv_fpr, w, st);
-    if (prec == DD_FP32) return compact ? nonlinear3<float, true, PH>(pl, u, inv_fpr, w, st)
-                                        : nonlinear3<float, false, PH>(pl, u, inv_fpr, w, st);
+                          const Work3& w, cudaStream_t st, const GradBufs* grads = nullptr) {
+    if (prec == DD_FP64) return compact ? nonlinear3<double, true, PH>(pl, u, inv_fpr, w, st, grads)
+                                        : nonlinear3<double, false, PH>(pl, u, inv_fpr, w, st, grads);
+    if (prec == DD_FP32) return compact ? nonlinear3<float, true, PH>(pl, u, inv_fpr, w, st, grads)
+                                        : nonlinear3<float, false, PH>(pl, u, inv_fpr, w, st, grads);
     if constexpr (PH == P3_HYDRO) {
         return compact ? nonlinear3<df64, true, PH>(pl, u, inv_fpr, w, st)
                        : nonlinear3<df64, false, PH>(pl, u, inv_fpr, w, st);
@@ -475,14 +475,16 @@ static int rhs3(const dd_plan* p, const double* params, const void* const* u, vo
     DD_CHECK_ARG(wb >= need, "workspace too small: %zu < %zu", wb, need);
     const double inv_fpr = p3_mhd(PH) ? inv_fpr_of(params) : 0.;
     Work3 w = make_work<PH>(g, work);
-    DD_TRY(nonlinear3_any<PH>(p, prec, false, u, inv_fpr, w, st));
+    GradBufs gb;
+    if (les) DD_TRY(les_grad_bufs(p, *les, prec, &gb));
+    DD_TRY(nonlinear3_any<PH>(p, prec, false, u, inv_fpr, w, st, les ? &gb : nullptr));
     ProjArgs pa{g, p->kx, p->ky, p->kz, inv_k2, inv_k2 != nullptr};
     CPtrs nc{}; Ptrs d{};
     for (int c = 0; c < P::NO; c++) nc.p[c] = work3_nc(prec, w, c);
     for (int c = 0; c < P::NF; c++) d.p[c] = deriv[c];
     if (les) {
         void* ncp[3] = {(void*)nc.p[0], (void*)nc.p[1], (void*)nc.p[2]};
-        DD_TRY(les_closure_add(p, *les, prec, false, u, ncp, st));
+        DD_TRY(les_closure_add(p, *les, prec, ncp, st));
     }
     if (zero_nonkept) {
         DD_KT("zero_nonkept3", st, launch(k_dealias3_all, dim3(ew_grid(g.kcount()), P::NF), 256, 0, st, g, d));
@@ -524,6 +526,8 @@ static int rk4_3(const dd_plan* p, const double* params, void* const* u, const d
     // FP32 transforms in divergence form without a closure: low-storage stages
     constexpr bool lo_ok = PH == P3_HYDRO_DIV || PH == P3_MHD_DIV;
     const bool lo = lo_ok && prec == DD_FP32 && les == nullptr;
+    GradBufs gb;
+    if (les) DD_TRY(les_grad_bufs(p, *les, prec, &gb));
     for (int s = 1; s <= 4; s++) {
         if constexpr (lo_ok) {
             if (lo) {
@@ -537,10 +541,10 @@ static int rk4_3(const dd_plan* p, const double* params, void* const* u, const d
                 continue;
             }
         }
-        DD_TRY(nonlinear3_any<PH>(p, prec, s > 1, s == 1 ? (const void* const*)u : ysc, inv_fpr, w, st));
+        DD_TRY(nonlinear3_any<PH>(p, prec, s > 1, s == 1 ? (const void* const*)u : ysc, inv_fpr, w, st, les ? &gb : nullptr));
         if (les) {
             void* ncp[3] = {(void*)a.nc.p[0], (void*)a.nc.p[1], (void*)a.nc.p[2]};
-            DD_TRY(les_closure_add(p, *les, prec, s > 1, s == 1 ? (const void* const*)u : ysc, ncp, st));
+            DD_TRY(les_closure_add(p, *les, prec, ncp, st));
         }
         a.stage = s; a.h = hs[s - 1]; a.w = ws[s - 1];
         for (int grp = 0; grp < P::NG; grp++)

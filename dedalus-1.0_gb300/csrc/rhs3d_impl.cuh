@@ -96,6 +96,22 @@ struct OpZInvCurl3 {
     }
 };
 
+// Pass 1 of the closed LES: fields 0..5 as above (velocity and vorticity) and the
+// nine gradients d_j u_a at field 6 + 3 a + j, for the closure's own x pass.
+template <typename T, bool COMPACT>
+struct OpZInvLes3 : OpZInvCurl3<T, COMPACT, 1> {
+    using Base = OpZInvCurl3<T, COMPACT, 1>;
+    static constexpr const char* name = "z_inv_les";
+    __device__ C<T> load(int fld, int kyc, int e, int ix) const {
+        if (fld < 6) return Base::load(fld, kyc, e, ix);
+        if (!kept_full(e, this->g.Nz, this->g.Mz)) return zero<T>();
+        const int ky_i = compact_to_full(kyc, this->g.Ny, this->g.Ky), j = (fld - 6) % 3;
+        const double k = j == 0 ? this->kx[ix] : j == 1 ? this->ky[ky_i] : this->kz[e];
+        const double2 v = ideriv(this->get((fld - 6) / 3, kyc, ky_i, e, ix), k);
+        return mk<T>((T)v.x, (T)v.y);
+    }
+};
+
 // ------------------------------------------------------------------ pass 3
 template <typename T>
 struct ProdHydro3 {
@@ -225,10 +241,20 @@ static Work3 make_work(const Geo3& g, void* base) {
                  (char*)base};
 }
 
+// Transform buffers of the nine velocity gradients of the closed LES: they are
+// transformed in the same z and y passes as the velocity and vorticity (a 64^3
+// pass takes a few microseconds: fifteen fields in one launch instead of six and nine,
+// and no kernel that forms the gradient spectra) and left in w2.
+struct GradBufs {
+    void* w1[9];
+    void* w2[9];
+};
+
 // ST = float (FP32 transforms only): compact stage states are read and the
 // compact products written as complex64 (the FP32 step's low-storage stages).
 template <typename T, bool COMPACT, int PH, typename ST = double>
-int nonlinear3(const dd_plan* pl, const void* const* u, double inv_fpr, const Work3& w, cudaStream_t st) {
+int nonlinear3(const dd_plan* pl, const void* const* u, double inv_fpr, const Work3& w, cudaStream_t st,
+               const GradBufs* grads = nullptr) {
     using P = Phys3<PH>;
     const Geo3& g = pl->g3;
     CPtrs uin{}; Ptrs w1{}, w2{}, nc{}; CPtrs w1c{}, w2c{};
@@ -239,10 +265,27 @@ int nonlinear3(const dd_plan* pl, const void* const* u, double inv_fpr, const Wo
         w1.p[f] = w.W1<T>(f); w1c.p[f] = w1.p[f];
         w2.p[f] = w.W2<T>(f); w2c.p[f] = w2.p[f];
     }
-    OpZInvCurl3<T, COMPACT, P::NG, p3_curl_inputs(PH), ST> a{g, uin, w1, TwSel<T>::z(pl), pl->kx, pl->ky, pl->kz};
-    DD_TRY((launch_pass_len<T, true, false, false>(g.Nz, a, g.Kx, g.Ky, P::NINV, st)));
+    int ninv = P::NINV;
+    bool first = true;
+    if constexpr (PH == P3_HYDRO && !std::is_same<T, df64>::value) {
+        if (grads) {
+            static_assert(P::NINV == 6 && P::NI == 6, "the gradients follow velocity and vorticity");
+            ninv = 15;
+            for (int f = 0; f < 9; f++) {
+                w1c.p[6 + f] = w1.p[6 + f] = grads->w1[f];
+                w2c.p[6 + f] = w2.p[6 + f] = grads->w2[f];
+            }
+            OpZInvLes3<T, COMPACT> a{{g, uin, w1, TwSel<T>::z(pl), pl->kx, pl->ky, pl->kz}};
+            DD_TRY((launch_pass_len<T, true, false, false>(g.Nz, a, g.Kx, g.Ky, ninv, st)));
+            first = false;
+        }
+    }
+    if (first) {
+        OpZInvCurl3<T, COMPACT, P::NG, p3_curl_inputs(PH), ST> a{g, uin, w1, TwSel<T>::z(pl), pl->kx, pl->ky, pl->kz};
+        DD_TRY((launch_pass_len<T, true, false, false>(g.Nz, a, g.Kx, g.Ky, ninv, st)));
+    }
     OpYInv3<T> b{g, w1c, w2, TwSel<T>::y(pl)};
-    DD_TRY((launch_pass_len<T, true, false, false>(g.Ny, b, g.Kx, g.Nz, P::NINV, st)));
+    DD_TRY((launch_pass_len<T, true, false, false>(g.Ny, b, g.Kx, g.Nz, ninv, st)));
     // products overwrite fields 0..NO-1 of W2 row by row (each block reads its rows first)
     if constexpr (PH == P3_HYDRO_DIV) {
         DD_TRY((launch_x_prod_len<T>("x_div", g.Nx, g.Nz * g.Ny, g.Kx, w2c, w2, 1, 0, 0, TwSel<T>::x(pl),
@@ -268,14 +311,14 @@ int nonlinear3(const dd_plan* pl, const void* const* u, double inv_fpr, const Wo
 // per arithmetic type, so the heavy transform kernels compile in parallel.
 #define DD_RHS3D_INSTANTIATE_PH(EXT, T, PH)                                                            \
     EXT template int nonlinear3<T, false, PH>(const dd_plan*, const void* const*, double, const Work3&,     \
-                                              cudaStream_t);                                            \
+                                              cudaStream_t, const GradBufs*);                           \
     EXT template int nonlinear3<T, true, PH>(const dd_plan*, const void* const*, double, const Work3&,      \
-                                             cudaStream_t);
+                                             cudaStream_t, const GradBufs*);
 #define DD_RHS3D_INSTANTIATE_LO(EXT, PH)                                                                \
     EXT template int nonlinear3<float, false, PH, float>(const dd_plan*, const void* const*, double,         \
-                                                         const Work3&, cudaStream_t);                        \
+                                                         const Work3&, cudaStream_t, const GradBufs*);       \
     EXT template int nonlinear3<float, true, PH, float>(const dd_plan*, const void* const*, double,          \
-                                                        const Work3&, cudaStream_t);
+                                                        const Work3&, cudaStream_t, const GradBufs*);
 // hydro forms and MHD forms, each compiled in its own translation unit; FP32
 // adds the low-storage stage variants of the divergence forms
 #define DD_RHS3D_INSTANTIATE_A(EXT, T) DD_RHS3D_INSTANTIATE_PH(EXT, T, P3_HYDRO) \
