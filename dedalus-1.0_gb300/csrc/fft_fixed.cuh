@@ -267,18 +267,22 @@ __device__ __forceinline__ void fx_dft(C<fx>* v) {
 // need 64 registers, so that 1024 threads fit an SM: at 256 points the y passes
 // of a 256^3 step took 248 / 150 us (forward / inverse) against 281 / 178 us for
 // two radix-16 passes (116 registers, 512 threads).  8-pencil tiles keep global
-// accesses at 128 bytes; 4 pencils took 327 / 182 us.  Forward schedules end
+// accesses at 128 bytes; 4 pencils took 327 / 182 us.  Wider tiles are padded more
+// where a row keeps few modes: with 8 pencils for 16 the y passes of 6 fields of
+// 128^3 (43 modes) take 43.5 / 42.1 us against 46.2 / 45.1, with 8 for 32 those of
+// 64^3 (22 modes) 8.6 / 8.5 us against 10.7 / 10.6, and with 16 for 64 those of 32^3
+// (11 modes) 6.3 / 6.5 us against 8.4 / 8.5.  Forward schedules end
 // with radix 8, whose outputs in the removed band are skipped, inverse ones begin
 // with it.
 template <int L> struct FxCfg;
 template <> struct FxCfg<8>   { static constexpr int P = 64, TPP = 1,  MB = 8, R[3] = {8, 1, 1}, RF[3] = {8, 1, 1}; };
 template <> struct FxCfg<16>  { static constexpr int P = 64, TPP = 4,  MB = 4, R[3] = {4, 4, 1}, RF[3] = {4, 4, 1}; };
 template <> struct FxCfg<24>  { static constexpr int P = 64, TPP = 4,  MB = 4, R[3] = {8, 3, 1}, RF[3] = {8, 3, 1}; };
-template <> struct FxCfg<32>  { static constexpr int P = 64, TPP = 4,  MB = 4, R[3] = {8, 4, 1}, RF[3] = {4, 8, 1}; };
+template <> struct FxCfg<32>  { static constexpr int P = 16, TPP = 4,  MB = 16, R[3] = {8, 4, 1}, RF[3] = {4, 8, 1}; };
 template <> struct FxCfg<48>  { static constexpr int P = 16, TPP = 16, MB = 4, R[3] = {4, 4, 3}, RF[3] = {4, 4, 3}; };
-template <> struct FxCfg<64>  { static constexpr int P = 32, TPP = 8,  MB = 4, R[3] = {8, 8, 1}, RF[3] = {8, 8, 1}; };
+template <> struct FxCfg<64>  { static constexpr int P = 8,  TPP = 8,  MB = 14, R[3] = {8, 8, 1}, RF[3] = {8, 8, 1}; };
 template <> struct FxCfg<96>  { static constexpr int P = 16, TPP = 12, MB = 5, R[3] = {8, 4, 3}, RF[3] = {8, 4, 3}; };
-template <> struct FxCfg<128> { static constexpr int P = 16, TPP = 16, MB = 4, R[3] = {8, 4, 4}, RF[3] = {4, 4, 8}; };
+template <> struct FxCfg<128> { static constexpr int P = 8,  TPP = 16, MB = 7, R[3] = {8, 4, 4}, RF[3] = {4, 4, 8}; };
 template <> struct FxCfg<192> { static constexpr int P = 8,  TPP = 24, MB = 5, R[3] = {8, 8, 3}, RF[3] = {8, 8, 3}; };
 template <> struct FxCfg<256> { static constexpr int P = 8,  TPP = 32, MB = 4, R[3] = {8, 8, 4}, RF[3] = {8, 4, 8}; };
 template <> struct FxCfg<512> { static constexpr int P = 8,  TPP = 64, MB = 2, R[3] = {8, 8, 8}, RF[3] = {8, 8, 8}; };
