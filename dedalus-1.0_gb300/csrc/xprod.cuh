@@ -89,12 +89,24 @@ struct ProdCfgT : ProdCfg<L, NI, NO> {
     static constexpr int min_blocks = std::is_same<T, df64>::value ? 5 : 1;   // __launch_bounds__
 };
 // FP64 (fixed-point transforms, a thread group per pencil): exactly the pencils
-// that the fields fill, as many rows as about 256 threads take, and registers for
-// 1024 threads per SM.
+// that the fields fill, the largest power of two of rows (2 to 16) whose pencils take
+// at most 192 threads, and registers for 1024 threads per SM.  Small blocks keep
+// fewer threads waiting at the block's barriers: on a 128^3 grid the MHD products (6
+// fields in, 8 out) take 190 us at 2 rows (128 threads), 201 at 4 and 235 at 8, hydro's
+// (3 and 5) 93 at 4 rows (160 threads), 99 at 6, 103 at 8 and 112 at 2; on 64^3 MHD
+// 27.0 at 4, 31.1 at 6 and 29.1 at 8, hydro 16.8 at 8 and 18.8 at 12.  256 threads for
+// the 2D products: alone they are 4% faster with 128, but an ensemble runs them
+// beside those of other lengths, where its step takes 2941 us against 2885 (128
+// uneven convection runs).
+constexpr int prod_rows_fx(int threads_per_row, int most) {
+    int q = 16;
+    while (q > 2 && q * threads_per_row > most) q /= 2;
+    return q;
+}
 template <int L, int NI, int NO>
 struct ProdCfgT<double, L, NI, NO> {
-    static constexpr int NM = NI > NO ? NI : NO, QF = (512 / (NM * FxRowTPP<L>::v)) & ~1;
-    static constexpr int Q = QF < 2 ? 2 : QF > 16 ? 16 : QF;
+    static constexpr int NM = NI > NO ? NI : NO;
+    static constexpr int Q = prod_rows_fx(NM * FxRowTPP<L>::v / 2, NM <= 4 ? 256 : 192);
     using SI = FxR<L, true, NI * Q / 2>;
     using SF = FxR<L, false, NO * Q / 2>;
     static constexpr int NT = ((SI::NT > SF::NT ? SI::NT : SF::NT) + 31) / 32 * 32;
