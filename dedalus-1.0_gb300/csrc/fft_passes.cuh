@@ -216,6 +216,17 @@ int launch_pass_sched(const Op& op, int npencil, int nslow, int nfield, cudaStre
     return DD_OK;
 }
 
+// Schedule of the FP32 passes over y and z: DefSched with fewer pencils per tile
+// at the lengths whose usual rows keep few modes (11, 16, 32 and 43; 32 or 64 pencils
+// did up to 75% of the work for padding) and whose 256-thread blocks left SMs idle:
+// FP32 hydro steps of 48^3 136 -> 131 us, 96^3 404 -> 376, 128^3 369 -> 339, MHD 128^3
+// 639 -> 596.  No gain at 64 points; at 256, 22 and 29 pencils were slower than 16.
+template <typename T, int L> struct NarrowSched { using S = DefSched<L>; };
+template <> struct NarrowSched<float, 32> { using S = Sched<32, 16, 64, 8, 4, 1>; };
+template <> struct NarrowSched<float, 48> { using S = Sched<48, 16, 64, 4, 4, 3>; };
+template <> struct NarrowSched<float, 96> { using S = Sched<96, 16, 64, 8, 4, 3>; };
+template <> struct NarrowSched<float, 128> { using S = Sched<128, 16, 128, 16, 8, 1>; };
+
 // The pass with the default schedule of its length.  An explicit one (pencils
 // per tile, threads, radix sequence) gives a small single-run grid enough
 // blocks to fill the GPU: a 128-point y pass of 43 kx pencils is 2 tiles of the
@@ -223,13 +234,18 @@ int launch_pass_sched(const Op& op, int npencil, int nslow, int nfield, cudaStre
 template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
 int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
     if constexpr (std::is_same<T, double>::value && RealRows<Op>::kind != 0) {
-        constexpr int TPP = FxRowTPP<L>::v, P = TPP >= 4 ? 256 / TPP : 64;   // about 256 threads
+        // 128 threads: no barriers between groups, and a block's shared memory is
+        // free sooner (192x128x256 there and back 504 us with 256, 497 with 128); 256
+        // at 512 points (64x128x512: 362 against 383)
+        constexpr int TPP = FxRowTPP<L>::v, P = TPP == 64 ? 4 : TPP >= 2 ? 128 / TPP : 64;
         return launch_pass_sched<T, FxR<L, INV, P>, INV, LD_E, ST_E, 1024 / (P * TPP)>(op, npencil, nslow, nfield, st, "");
     } else if constexpr (std::is_same<T, double>::value)
         return launch_pass_sched<T, FxS<L, INV>, INV, LD_E, ST_E, FxCfg<L>::MB>(op, npencil, nslow, nfield, st, "");
-    else   // FP32 inverse passes at 256 points: 5 blocks (48 registers) gain 4% on 4, forward ones spill
-        return launch_pass_sched<T, DefSched<L>, INV, LD_E, ST_E, (std::is_same<T, float>::value && L == 256 && INV ? 5 : 0)>(
+    else {   // FP32 inverse passes at 256 points: 5 blocks (48 registers) gain 4% on 4, forward ones spill
+        using S = std::conditional_t<LD_E || ST_E, DefSched<L>, typename NarrowSched<T, L>::S>;
+        return launch_pass_sched<T, S, INV, LD_E, ST_E, (std::is_same<T, float>::value && L == 256 && INV ? 5 : 0)>(
             op, npencil, nslow, nfield, st, "");
+    }
 }
 
 // Small-tile schedules (4 pencils, 16 threads each) for single-run 2D grids.
