@@ -248,17 +248,28 @@ int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t s
     }
 }
 
-// Small-tile schedules (4 pencils, 16 threads each) for single-run 2D grids.
-template <int L> struct SmallSched;
-template <> struct SmallSched<64> { using S = Sched<64, 4, 64, 4, 4, 4>; };
-template <> struct SmallSched<128> { using S = Sched<128, 4, 64, 8, 4, 4>; };
+// Small-tile schedules for single-run 2D grids: 4 pencils of 16 threads, and at
+// 256 and 512 points 2 pencils of the usual threads and radices (a 512-point y pass of
+// 171 kx pencils of 3 fields is 66 tiles of 8, or 258 of 2, for 152 SMs: a 512^2
+// convection step takes 181 us, 195 with 8; a 512^2 hydro step 138, 146 with 8).
+template <typename T, int L, bool INV> struct SmallSched { using S = Sched<L, 2, 2 * DefSched<L>::TPP, DefSched<L>::R1, DefSched<L>::R2, DefSched<L>::R3>; };
+template <int L, bool INV> struct SmallSched<double, L, INV> { using S = FxS<L, INV, 2>; };
+template <typename T, bool INV> struct SmallSched<T, 64, INV> { using S = Sched<64, 4, 64, 4, 4, 4>; };
+template <typename T, bool INV> struct SmallSched<T, 128, INV> { using S = Sched<128, 4, 64, 8, 4, 4>; };
+template <bool INV> struct SmallSched<double, 64, INV> { using S = Sched<64, 4, 64, 4, 4, 4>; };
+template <bool INV> struct SmallSched<double, 128, INV> { using S = Sched<128, 4, 64, 8, 4, 4>; };
 
 // Launch a pass with the small-tile schedule when one exists for length L;
 // returns 1 (not launched) otherwise.
 template <typename T, bool INV, bool LD_E, bool ST_E, class Op>
 int launch_pass_small(int L, const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
-    if (L == 64) return launch_pass_sched<T, typename SmallSched<64>::S, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st);
-    if (L == 128) return launch_pass_sched<T, typename SmallSched<128>::S, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st);
+#define DD_SMALL(N) \
+    if (L == N) return launch_pass_sched<T, typename SmallSched<T, N, INV>::S, INV, LD_E, ST_E>(op, npencil, nslow, nfield, st);
+    DD_SMALL(64)
+    DD_SMALL(128)
+    DD_SMALL(256)
+    DD_SMALL(512)
+#undef DD_SMALL
     return 1;
 }
 

@@ -187,11 +187,11 @@ int nonlinear2(const dd_plan* pl, const Work2& w, const void* const* st, int64_t
         if constexpr (std::is_same<ST, float>::value) nc.p[f] = w.NCf(f);
         else nc.p[f] = w.NC<T>(f);
     }
-    // one run of a 64- or 128-point grid: small tiles, so that the y passes
-    // have enough blocks (the default 32-pencil tiles give 2 per field)
+    // one run: small tiles where they exist, so that the y passes have enough
+    // blocks (at 128 points the default tiles give 2 to 6 per field)
     // (a tuned tile variant, set on the plan, takes precedence)
     const int yv = pl->sched_y2d;
-    const bool small = yv == 0 && w.nrun == 1 && (g.Ny == 64 || g.Ny == 128);
+    const bool small = yv == 0 && w.nrun == 1;
     OpYInvPhys2<T, COMPACT, PHYS, ST> a{g, sin, st_rs, wo, (int64_t)w.w, TwSel<T>::y(pl), pl->kx, pl->ky};
     int rc = 1;
     if (yv) rc = launch_pass_variant<T, true, true, false>(g.Ny, yv, a, g.Kx, w.nrun, PH::NI, s);
