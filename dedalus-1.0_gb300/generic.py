@@ -1,6 +1,9 @@
 """Reference-ordered right-hand sides on the GPU, for the physics branches the
 fused kernels do not cover: the shearing box (``FourierShearRepresentation``
 with ``shear_rate`` != 0), rotation (``Omega``), 3D Boussinesq and 2D MHD.
+Rotation and 3D Boussinesq without shear, on axes of 16 to 512 points, run as
+one library call with the same operand order (``dd_advect_rhs3d``,
+``_advect_rhs``); everything else runs operator by operator.
 
 The operator helpers are the reference's (dedalus/physics/physics.py:
 ``divX`` 180-195, ``XgradY`` 197-228, ``XconstcrossY`` 266-307,
