@@ -53,6 +53,7 @@ SIGNATURES = {
     "dd_etd1": [I, P, P, P, P, D, I64, P],
     "dd_etd2rk1": [I, P, P, P, P, P, D, I64, P],
     "dd_etd2rk2": [I, P, P, P, P, P, D, I64, P],
+    "dd_etd_fields": [I, I, I, PP, PP, PP, PP, PP, D, I64, P],
     "dd_phi_table": [I, D, I, D, I, P, P],
     "dd_hydro3d_workspace_size": [P, I, ctypes.POINTER(SZ)],
     "dd_hydro3d_rhs": [P, PP, PP, P, I, I, P, SZ, P],

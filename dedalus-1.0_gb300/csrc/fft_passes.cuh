@@ -229,8 +229,8 @@ template <> struct NarrowSched<float, 128> { using S = Sched<128, 16, 128, 16, 8
 
 // The pass with the default schedule of its length.  An explicit one (pencils
 // per tile, threads, radix sequence) gives a small single-run grid enough
-// blocks to fill the GPU: a 128-point y pass of 43 kx pencils is 2 tiles of the
-// default 32 pencils, but 11 tiles of 4.
+// blocks to fill the GPU: a 128-point y pass of 43 kx pencils is 6 tiles of the
+// default 8 pencils (FP32: 3 of 16), but 11 tiles of 4.
 template <typename T, int L, bool INV, bool LD_E, bool ST_E, class Op>
 int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t st) {
     if constexpr (std::is_same<T, double>::value && RealRows<Op>::kind != 0) {

@@ -188,7 +188,7 @@ int nonlinear2(const dd_plan* pl, const Work2& w, const void* const* st, int64_t
         else nc.p[f] = w.NC<T>(f);
     }
     // one run: small tiles where they exist, so that the y passes have enough
-    // blocks (at 128 points the default tiles give 2 to 6 per field)
+    // blocks (at 128 points the default tiles give 3 to 6 per field)
     // (a tuned tile variant, set on the plan, takes precedence)
     const int yv = pl->sched_y2d;
     const bool small = yv == 0 && w.nrun == 1;

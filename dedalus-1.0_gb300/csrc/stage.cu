@@ -3,6 +3,7 @@
 // phi-function table used by the fused timesteppers.
 #include "dd_common.cuh"
 #include "etd.cuh"
+#include "geometry.cuh"
 
 namespace dd {
 
@@ -54,6 +55,54 @@ __global__ void k_etd2rk2(const double2* s, double2* o, const double2* __restric
         if (Z != 0.) etd_phis<NDIM>(Z, f0, f1, f2);
         o[i] = etd2rk2_entry(s[i], d1[i], d2[i], Z, f0, f1, f2, dt);
     }
+}
+
+// One stage update of up to ETD_FIELDS fields: SCHEME 0 etd1, 1 etd2rk1, 2 etd2rk2.
+// Bound by the FP64 pipe (exp and a polynomial or two divisions per entry, 43-48 us
+// per field of 64^3), so a thread takes one entry of all fields and evaluates the
+// phi functions anew only where the factor differs from the field before (the
+// components of u share theirs): the 8 updates of a 64^3 rotating Boussinesq
+// RK2trap step took 365 us of 515 as one launch per field, and take 107 of 281 as
+// two launches.  Blocks of 128 threads: 64^3 is
+// 6.9 of them per SM, where 3.5 of 256 leave half a wave idle.
+constexpr int ETD_FIELDS = 6;
+struct EtdFields {
+    int nf;
+    const double2* s[ETD_FIELDS];
+    double2* o[ETD_FIELDS];
+    const double2* d1[ETD_FIELDS];
+    const double2* d2[ETD_FIELDS];
+    const double* intf[ETD_FIELDS];
+};
+
+template <int NDIM, int SCHEME>
+__global__ void __launch_bounds__(128) k_etd_fields(EtdFields a, double dt, int64_t n) {
+    grid_wait();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double Zp = 0., f0 = 1., f1 = 1., f2 = 0.5;
+#pragma unroll 1
+        for (int f = 0; f < a.nf; f++) {
+            const double Z = rmul(pick_ptr<ETD_FIELDS>(a.intf, f)[i], dt);
+            const double2 s = pick_ptr<ETD_FIELDS>(a.s, f)[i], d1 = pick_ptr<ETD_FIELDS>(a.d1, f)[i];
+            if (Z != Zp) {
+                if (Z != 0.) etd_phis<NDIM>(Z, f0, f1, f2);
+                Zp = Z;
+            }
+            double2* o = pick_ptr<ETD_FIELDS>(a.o, f);
+            if (SCHEME == 0) o[i] = etd1_entry(s, d1, Z, f0, f1, dt);
+            else if (SCHEME == 1) o[i] = etd2rk1_entry(s, d1, pick_ptr<ETD_FIELDS>(a.d2, f)[i], Z, f2, dt);
+            else o[i] = etd2rk2_entry(s, d1, pick_ptr<ETD_FIELDS>(a.d2, f)[i], Z, f0, f1, f2, dt);
+        }
+    }
+}
+
+template <int NDIM>
+static void launch_etd_fields(int scheme, const EtdFields& a, double dt, int64_t n, cudaStream_t st) {
+    const int64_t nb = (n + 127) / 128;
+    const unsigned b = (unsigned)(nb > 152 * 64 ? 152 * 64 : nb);
+    if (scheme == 0) DD_KT("etd1_fields", st, launch(k_etd_fields<NDIM, 0>, b, 128, 0, st, a, dt, n));
+    else if (scheme == 1) DD_KT("etd2rk1_fields", st, launch(k_etd_fields<NDIM, 1>, b, 128, 0, st, a, dt, n));
+    else DD_KT("etd2rk2_fields", st, launch(k_etd_fields<NDIM, 2>, b, 128, 0, st, a, dt, n));
 }
 
 // table[q] = {Z, f0, f1, f2} for integer squared wavenumber q with
@@ -141,6 +190,35 @@ int dd_etd2rk2(int ndim, const void* start, void* output, const void* deriv1, co
         DD_KT("etd2rk23", st, launch(k_etd2rk2<3>, ew_blocks(n), 256, 0, st, (const double2*)start, (double2*)output, (const double2*)deriv1,
                                                    (const double2*)deriv2, intfactor, dt, n));
     DD_LAUNCH_CHECK();
+    return DD_OK;
+}
+
+int dd_etd_fields(int ndim, int scheme, int nf, const void* const* start, void* const* output,
+                  const void* const* deriv1, const void* const* deriv2, const void* const* intfactor, double dt,
+                  int64_t n, void* stream) {
+    DD_CHECK_ARG(start && output && deriv1 && intfactor, "dd_etd_fields: null pointer");
+    DD_CHECK_ARG(ndim == 2 || ndim == 3, "dd_etd_fields: ndim must be 2 or 3");
+    DD_CHECK_ARG(scheme >= 0 && scheme <= 2, "dd_etd_fields: scheme must be 0, 1 or 2");
+    DD_CHECK_ARG(scheme == 0 || deriv2, "dd_etd_fields: null pointer");
+    DD_CHECK_ARG(nf >= 0 && n >= 0, "dd_etd_fields: negative size");
+    for (int f = 0; f < nf; f++)
+        DD_CHECK_ARG(start[f] && output[f] && deriv1[f] && intfactor[f] && (scheme == 0 || deriv2[f]),
+                     "dd_etd_fields: null pointer of field %d", f);
+    if (n == 0) return DD_OK;
+    for (int f0 = 0; f0 < nf; f0 += ETD_FIELDS) {
+        EtdFields a{};
+        a.nf = nf - f0 < ETD_FIELDS ? nf - f0 : ETD_FIELDS;
+        for (int f = 0; f < a.nf; f++) {
+            a.s[f] = (const double2*)start[f0 + f];
+            a.o[f] = (double2*)output[f0 + f];
+            a.d1[f] = (const double2*)deriv1[f0 + f];
+            a.d2[f] = scheme == 0 ? nullptr : (const double2*)deriv2[f0 + f];
+            a.intf[f] = (const double*)intfactor[f0 + f];
+        }
+        if (ndim == 2) launch_etd_fields<2>(scheme, a, dt, n, (cudaStream_t)stream);
+        else launch_etd_fields<3>(scheme, a, dt, n, (cudaStream_t)stream);
+        DD_LAUNCH_CHECK();
+    }
     return DD_OK;
 }
 

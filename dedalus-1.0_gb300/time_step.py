@@ -39,6 +39,18 @@ def _neg_if(comp):
     return t
 
 
+def _etd(scheme, rows, dt):
+    """``dd_etd1`` (scheme 0), ``dd_etd2rk1`` (1) or ``dd_etd2rk2`` (2) on the rows (start, output,
+    derivatives..., -integrating factor), one call for rows of one shape."""
+    groups = {}
+    for row in rows:
+        groups.setdefault(row[0].shape, []).append(row)
+    for shape, rows in groups.items():
+        p = [(ctypes.c_void_p * len(rows))(*[t.data_ptr() for t in col]) for col in zip(*rows)]
+        _lib.call("dd_etd_fields", len(shape), scheme, len(rows), p[0], p[1], p[2],
+                  p[3] if scheme else None, p[-1], float(dt), rows[0][0].numel(), current_stream())
+
+
 class TimeStepBase:
     """time_step.py:48-179."""
 
@@ -155,6 +167,7 @@ class RK2mid(RKBase):
         data2, deriv1, deriv2 = self.data2, self.deriv1, self.deriv2
         st = current_stream()
         self.RHS.RHS(data, deriv1)
+        rows = []
         for f in data.fields.keys():
             for c in range(data[f].ncomp):
                 d1 = deriv1[f][c]
@@ -162,10 +175,11 @@ class RK2mid(RKBase):
                 if d1.integrating_factor is None:
                     _lib.call("dd_euler", dptr(s), dptr(o), dptr(k1), dt / 2., s.numel(), st)
                 else:
-                    _lib.call("dd_etd1", s.dim(), dptr(s), dptr(o), dptr(k1), dptr(_neg_if(d1)), dt / 2.,
-                              s.numel(), st)
+                    rows.append((s, o, k1, _neg_if(d1)))
+        _etd(0, rows, dt / 2.)
         data2.set_time(data.time + dt / 2.)
         self.RHS.RHS(data2, deriv2)
+        rows = []
         for f in data.fields.keys():
             for c in range(data[f].ncomp):
                 d1 = deriv1[f][c]
@@ -173,8 +187,8 @@ class RK2mid(RKBase):
                 if d1.integrating_factor is None:
                     _lib.call("dd_euler", dptr(s), dptr(s), dptr(k2), float(dt), s.numel(), st)
                 else:
-                    _lib.call("dd_etd2rk2", s.dim(), dptr(s), dptr(s), dptr(k1), dptr(k2), dptr(_neg_if(d1)),
-                              float(dt), s.numel(), st)
+                    rows.append((s, s, k1, k2, _neg_if(d1)))
+        _etd(2, rows, dt)
         data.set_time(data.time + dt)
         self._finish(dt)
 
@@ -192,6 +206,7 @@ class RK2trap(RKBase):
         deriv1, deriv2 = self.deriv1, self.deriv2
         st = current_stream()
         self.RHS.RHS(data, deriv1)
+        rows = []
         for f in data.fields.keys():
             for c in range(data[f].ncomp):
                 d1 = deriv1[f][c]
@@ -199,10 +214,11 @@ class RK2trap(RKBase):
                 if d1.integrating_factor is None:
                     _lib.call("dd_euler", dptr(s), dptr(s), dptr(k1), float(dt), s.numel(), st)
                 else:
-                    _lib.call("dd_etd1", s.dim(), dptr(s), dptr(s), dptr(k1), dptr(_neg_if(d1)), float(dt),
-                              s.numel(), st)
+                    rows.append((s, s, k1, _neg_if(d1)))
+        _etd(0, rows, dt)
         data.set_time(data.time + dt)
         self.RHS.RHS(data, deriv2)
+        rows = []
         for f in data.fields.keys():
             for c in range(data[f].ncomp):
                 d1 = deriv1[f][c]
@@ -215,8 +231,8 @@ class RK2trap(RKBase):
                     _lib.call("dd_scale_add", dptr(k1), dptr(self._diff), -1.0, 1, s.numel(), st)
                     _lib.call("dd_euler", dptr(s), dptr(s), dptr(self._diff), dt / 2., s.numel(), st)
                 else:
-                    _lib.call("dd_etd2rk1", s.dim(), dptr(s), dptr(s), dptr(k1), dptr(k2), dptr(_neg_if(d1)),
-                              float(dt), s.numel(), st)
+                    rows.append((s, s, k1, k2, _neg_if(d1)))
+        _etd(1, rows, dt)
         self._finish(dt)
 
 

@@ -150,6 +150,12 @@ int dd_etd2rk1(int ndim, const void* start, void* output, const void* deriv1, co
                const double* intfactor, double dt, int64_t n, void* stream);
 int dd_etd2rk2(int ndim, const void* start, void* output, const void* deriv1, const void* deriv2,
                const double* intfactor, double dt, int64_t n, void* stream);
+/* One of these updates (scheme 0: etd1, 1: etd2rk1, 2: etd2rk2; deriv2 unused by etd1)
+ * on nf fields of n entries each: the same results as nf calls.  No output may be
+ * an input of another field. */
+int dd_etd_fields(int ndim, int scheme, int nf, const void* const* start, void* const* output,
+                  const void* const* deriv1, const void* const* deriv2, const void* const* intfactor, double dt,
+                  int64_t n, void* stream);
 
 /* phi-function table for integer squared wavenumbers q = 0..qmax:
  * table[q] = {Z, f0(Z), f1(Z), f2(Z)} (4 doubles) with Z = -(nu q^vo) h, the

@@ -1,6 +1,6 @@
 """Single 2D runs with 256- and 512-point y passes (tiles of 2 pencils) on rows
 that keep an odd and an even number of modes, against the CPU oracle.  Tolerances:
-those of the other 2D right-hand sides, 1e-12 relative L2 in FP64 and 1e-4 with
+those of the other right-hand sides, 1e-12 relative L2 in FP64 and 1e-4 with
 FP32 transforms.
 """
 import numpy as np
