@@ -60,8 +60,10 @@ struct AdvArgs {
     double om[3], gg, alpha_t, beta;
 };
 
-// All modes of the full layout, one per thread.
-__global__ void __launch_bounds__(256) k_advect_tail3(AdvArgs a) {
+// All modes of the full layout, one per thread, bound by the FP64 pipe.  128-thread
+// blocks: 64^3 is 6.9 per SM, where 3.5 of 256 threads leave half a wave idle (27 us
+// at 64^3; 31 with those and a predicated buoyancy addition per axis).
+__global__ void __launch_bounds__(128) k_advect_tail3(AdvArgs a) {
     grid_wait();
     const Geo3& g = a.g;
     const int64_t n = g.kcount();
@@ -98,13 +100,13 @@ __global__ void __launch_bounds__(256) k_advect_tail3(AdvArgs a) {
         if (a.ns == 4) {        // physics.py:688-708
             const double2 T = ((const double2*)a.y.p[3])[i];
             const double2 b = make_double2(rmul(rmul(T.x, a.gg), a.alpha_t), rmul(rmul(T.y, a.gg), a.alpha_t));
-            double2 ud = u[0];
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-                if (c == a.dir) {
-                    N[c] = make_double2(radd(N[c].x, b.x), radd(N[c].y, b.y));
-                    ud = u[c];
-                }
+            // one addition and selects: a predicated one per axis takes the FP64 pipe three times
+            const double2 ud = a.dir == 0 ? u[0] : a.dir == 1 ? u[1] : u[2];
+            double2 nd = a.dir == 0 ? N[0] : a.dir == 1 ? N[1] : N[2];
+            nd = make_double2(radd(nd.x, b.x), radd(nd.y, b.y));
+            if (a.dir == 0) N[0] = nd;
+            else if (a.dir == 1) N[1] = nd;
+            else N[2] = nd;
             ((double2*)a.d.p[3])[i] = make_double2(rsub(N[3].x, rmul(ud.x, a.beta)), rsub(N[3].y, rmul(ud.y, a.beta)));
         }
         // pressure projection (physics.py:588-599, 407-416)
@@ -153,7 +155,7 @@ static int advect_rhs3d(const dd_plan* p, AdvArgs& a, void* work, size_t wb, cud
     OpZFwdCompact3<double> zf{g, w1c, nc, p->tw64_z};
     DD_TRY((launch_pass_len<double, false, false, false>(g.Nz, zf, g.Kx, g.Ky, NS, st)));
     const int64_t n = g.kcount();
-    DD_KT("advect_tail3", st, launch(k_advect_tail3, (unsigned)(n > 152 * 16 * 256 ? 152 * 16 : (n + 255) / 256), 256, 0, st, a));
+    DD_KT("advect_tail3", st, launch(k_advect_tail3, (unsigned)(n > 152 * 32 * 128 ? 152 * 32 : (n + 127) / 128), 128, 0, st, a));
     DD_LAUNCH_CHECK();
     return DD_OK;
 }

@@ -62,7 +62,7 @@ __global__ void k_etd2rk2(const double2* s, double2* o, const double2* __restric
 // per field of 64^3), so a thread takes one entry of all fields and evaluates the
 // phi functions anew only where the factor differs from the field before (the
 // components of u share theirs): the 8 updates of a 64^3 rotating Boussinesq
-// RK2trap step took 365 us of 515 as one launch per field, and take 107 of 281 as
+// RK2trap step took 365 us of 515 as one launch per field, and take 107 of 270 as
 // two launches.  Blocks of 128 threads: 64^3 is
 // 6.9 of them per SM, where 3.5 of 256 leave half a wave idle.
 constexpr int ETD_FIELDS = 6;
