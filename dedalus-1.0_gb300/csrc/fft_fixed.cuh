@@ -636,8 +636,9 @@ __device__ __forceinline__ void fx_group_later(C<double>* tile, C<fx> (&v)[fx_bp
 // c2r: two half spectra A, B (kx < Kx) into the packed sequence Z = A + iB in
 // fixed point (each mode is loaded and converted once for both of its places in
 // Z), then the inverse transform, whose real and imaginary parts are the two rows
-// (doubles in the tile).  get(k, A, B) loads; the imaginary parts at kx = 0 are
-// dropped, as a c2r transform does.
+// (doubles in the tile).  get(k, A, B) loads; the imaginary parts at kx = 0 and
+// kx = L/2 are dropped, as a c2r transform does.  kx = L/2 is kept by plans with
+// Kx = L/2 + 1 only, which the 2/3 rule (PRUNE) never is.
 template <class S, bool PRUNE, class Get>
 __device__ __forceinline__ void fx_group_c2r(C<double>* tile, const int4* tw, int p, int jt, int Kx, unsigned* red, Get get) {
     constexpr int L = S::L, H = L / 2, TPP = S::TPP, NPT = (H + TPP - 1) / TPP, R1 = S::R1, NB1 = L / R1;
@@ -645,7 +646,7 @@ __device__ __forceinline__ void fx_group_c2r(C<double>* tile, const int4* tw, in
     C<fx>* ft = reinterpret_cast<C<fx>*>(tile);
     FxScale sc;
     {
-        C<double> AB[NPT][2];
+        C<double> AB[NPT][2], last = mk<double>(0., 0.);   // last: real parts of both rows at kx = L/2
         unsigned h = 0;
 #pragma unroll
         for (int i = 0; i < NPT; i++) {
@@ -654,18 +655,33 @@ __device__ __forceinline__ void fx_group_c2r(C<double>* tile, const int4* tw, in
             if (k < Kx) get(k, AB[i][0], AB[i][1]);
             if (k == 0) { AB[i][0].y = 0.; AB[i][1].y = 0.; }
         }
+        if constexpr (!PRUNE) {
+            if (Kx > H && jt == 0) {
+                C<double> A = mk<double>(0., 0.), B = mk<double>(0., 0.);
+                get(H, A, B);
+                last = mk<double>(A.x, B.x);
+                h = fx_max(h, last);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < NPT; i++) h = fx_max(fx_max(h, AB[i][0]), AB[i][1]);
         sc = fx_scale(fx_group_max<TPP>(h, p, red) >> 1);
-        if (sc.rare) fx_scale_all<2 * NPT>(&AB[0][0], fx_pre(sc.rare));
+        if (sc.rare) {
+            fx_scale_all<2 * NPT>(&AB[0][0], fx_pre(sc.rare));
+            if constexpr (!PRUNE) fx_scale_all<1>(&last, fx_pre(sc.rare));
+        }
         const int K = fx_kin<S>(sc.e2, true);
+        C<fx> lastf = mk<fx>(0, 0);
+        if constexpr (!PRUNE) {
+            if (Kx > H) lastf = fx_in(last, K);
+        }
 #pragma unroll
         for (int i = 0; i < NPT; i++) {
             const int k = jt + TPP * i;
             if (H % TPP != 0 && k >= H) continue;
             const C<fx> a = fx_in(AB[i][0], K), b = fx_in(AB[i][1], K);
             ft[S::off(k) + p] = mk<fx>(a.x - b.y, a.y + b.x);
-            ft[S::off(k == 0 ? H : L - k) + p] = k == 0 ? mk<fx>(0, 0) : mk<fx>(a.x + b.y, b.x - a.y);
+            ft[S::off(k == 0 ? H : L - k) + p] = k == 0 ? lastf : mk<fx>(a.x + b.y, b.x - a.y);
         }
     }
     fx_group_sync<TPP>(p);

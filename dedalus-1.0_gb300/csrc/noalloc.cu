@@ -12,8 +12,8 @@
 // Limits and rules, for the caller:
 //  * The buffer holds DD_NOALLOC_SCRATCH_BYTES (4 MiB).  That covers one FP64
 //    field up to 64^3 in 3D and up to 512^2 in 2D, with or without 2/3
-//    dealiasing (the Nyquist modes are never kept, so a 64^3 plan needs at
-//    most 4.16 MB, 2.4 MB with 2/3 dealiasing); larger grids are rejected
+//    dealiasing (a 64^3 plan that does not keep kx = 32 needs at most 4.16
+//    MB, 2.4 MB with 2/3 dealiasing); larger grids are rejected
 //    with DD_ERR_UNSUPPORTED and a message giving the bytes they need.
 //  * Every GPU that loads the library holds the 4 MiB until the process exits.
 //  * Every call looks up the buffer's device address on the current device

@@ -67,6 +67,8 @@ int dd_timing_report(char* buf, size_t len);
  * order: kx[Nx/2+1], ky[Ny], kz[Nz] (3D) or kx[Nx/2+1], ky[Ny] (2D), on the
  * host.  mx, my, mz give the largest kept |mode index| per axis after
  * dealiasing (representations.py:359-408): kept modes are 0..m and N-m..N-1.
+ * mx may be Nx/2 (the backward transforms then take the real part at kx = Nx/2, as
+ * they do at kx = 0); 2 my + 1 <= Ny and 2 mz + 1 <= Nz.
  * Fails with DD_ERR_UNSUPPORTED for other sizes.
  */
 int dd_plan_create(int ndim, const int64_t* xshape, const double* kx, const double* ky,
@@ -108,8 +110,8 @@ int dd_fft_c2r(const dd_plan* plan, int nfield, const void* const* k, double* co
  * synchronisation are not allowed, or the caller's host language has no
  * device allocator).  Intermediates live in a 4 MiB static device buffer in
  * the library image (held on every GPU that loads the library): grids up to
- * 64^3 (3D) and 512^2 (2D), with or without 2/3 dealiasing (Nyquist modes are
- * never kept); larger ones return DD_ERR_UNSUPPORTED.  Each call looks the buffer
+ * 64^3 (3D) and 512^2 (2D), with or without 2/3 dealiasing, where mx < Nx/2;
+ * larger ones return DD_ERR_UNSUPPORTED.  Each call looks the buffer
  * up on the current device (cudaGetSymbolAddress); the first call on a device
  * should come before any stream capture.  The plan must belong to the current
  * device (DD_ERR_INVALID otherwise).  All calls share the buffer: calls whose
