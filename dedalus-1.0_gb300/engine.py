@@ -36,7 +36,8 @@ class Plan:
         self.kshape = kgrid.kspace_shape(list(self.xshape))
         self.mx, self.my, self.mz = kgrid.kept_bounds(self.xshape, self.length, dealiasing)
         self.kx, self.ky, self.kz = kgrid.k_tables(self.xshape, self.length)
-        self.integer_k = kgrid.integer_k(self.xshape, self.length)
+        self.integer_k2_max = kgrid.integer_k2_max(self.xshape, self.length)
+        self.integer_k = self.integer_k2_max is not None
         shape = (ctypes.c_int64 * self.ndim)(*self.xshape)
         h = ctypes.c_void_p()
         with torch.cuda.device(self.device):

@@ -99,9 +99,25 @@ def k_tables(xshape, length):
     return kx, ky, kz
 
 
-def integer_k(xshape, length):
-    """True when every wavenumber is an exact integer (length 2 pi axes)."""
+# Squared wavenumbers up to which the steps look 1/k^2 and the phi functions up in
+# tables of one entry per integer k^2: 2^22 entries are 128 MiB per phi table, and
+# the kernels that form k^2 in single precision need it below 2^24.
+INTEGER_K2_LIMIT = 1 << 22
+
+
+def integer_k2_max(xshape, length):
+    """Largest |k|^2 of the grid when every wavenumber is an exact integer (sides 2 pi / m)
+    and it is at most INTEGER_K2_LIMIT, otherwise None."""
+    q = 0
     for t in k_tables(xshape, length):
-        if t is not None and not np.array_equal(t, np.round(t)):
-            return False
-    return True
+        if t is None:
+            continue
+        if not np.array_equal(t, np.round(t)):
+            return None
+        q += int(np.abs(t).max()) ** 2
+    return q if q <= INTEGER_K2_LIMIT else None
+
+
+def integer_k(xshape, length):
+    """True when the q tables cover this grid (integer_k2_max)."""
+    return integer_k2_max(xshape, length) is not None

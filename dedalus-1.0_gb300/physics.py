@@ -90,7 +90,7 @@ class Physics:
         key = ('inv_k2', id(plan))
         t = self._tables.get(key)
         if t is None:
-            qmax = int(sum((n // 2) ** 2 for n in plan.xshape))
+            qmax = plan.integer_k2_max
             q = np.arange(qmax + 1, dtype=np.float64)
             q[0] = 1.
             t = torch.from_numpy(1.0 / q).to(plan.device)
@@ -102,7 +102,7 @@ class Physics:
         key = ('phi', id(plan), float(nu), int(vo), float(h))
         t = self._tables.get(key)
         if t is None:
-            qmax = int(sum((n // 2) ** 2 for n in plan.xshape))
+            qmax = plan.integer_k2_max
             t = torch.empty((qmax + 1, 4), dtype=torch.float64, device=plan.device)
             _lib.call("dd_phi_table", plan.ndim, float(nu), int(vo), float(h), qmax, dptr(t), current_stream())
             if len(self._tables) > 64:

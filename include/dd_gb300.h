@@ -171,7 +171,9 @@ int dd_phi_table(int ndim, double nu, int viscosity_order, double h, int qmax, v
  * form; equal on the kept modes to roundoff).  u and deriv are 3 component
  * k arrays (x, y, z order, full reference layout).  inv_k2 is an optional
  * device table 1/q for integer squared wavenumbers q (q = 0 -> 1); pass it
- * when every wavenumber is an integer (length-2 pi axes), else NULL.
+ * when every wavenumber is an integer (sides 2 pi / m) and |k|^2 < 2^24, else
+ * NULL.  It and the phi tables given with it need an entry for every q up to the
+ * largest |k|^2 of the grid, Nyquist modes included.
  * zero_nonkept != 0 also writes zeros to the non-kept entries of deriv (the
  * reference zeroes deriv first, physics.py:140-142).  precision selects FP64
  * or FP32 transform/product arithmetic; the projection is FP64. */
