@@ -3,7 +3,8 @@ fused kernels do not cover: the shearing box (``FourierShearRepresentation``
 with ``shear_rate`` != 0), rotation (``Omega``), 3D Boussinesq and 2D MHD.
 Rotation and 3D Boussinesq without shear, on axes of 16 to 512 points, run as
 one library call with the same operand order (``dd_advect_rhs3d``,
-``_advect_rhs``); everything else runs operator by operator.
+``_advect_rhs``), unless a subclass or an instance has operators, a representation
+or a k^2 of its own (``_advect_fused``); everything else runs operator by operator.
 
 The operator helpers are the reference's (dedalus/physics/physics.py:
 ``divX`` 180-195, ``XgradY`` 197-228, ``XconstcrossY`` 266-307,
@@ -29,6 +30,7 @@ import torch
 
 from . import _lib
 from .engine import current_stream, dptr
+from .representations import FourierRepresentation
 
 
 # ----------------------------------------------------------- elementwise ops
@@ -225,9 +227,14 @@ class ReferenceOrderRHS:
     # ------------------------------------------------- right-hand sides
     def _advect_fused(self, data):
         """True when dd_advect_rhs3d covers this 3D right-hand side: a static
-        basis (no shear) and axis lengths of the fused passes."""
+        basis (no shear), axis lengths of the fused passes, and the operators, the
+        representation and k^2 that the call stands for (a k2 set on the object
+        before its first right-hand side is used by laplace_solve only)."""
         return (self.ndim == 3 and not self._shear and self._representation._static_k
-                and min(self.plan(data).xshape) >= 16)
+                and min(self.plan(data).xshape) >= 16
+                and (self.k2 is None or self.laplace_k2 == 'current')
+                and all(getattr(getattr(self, n), '__func__', None) is f for n, f in _OPERATORS)
+                and all(getattr(self._representation, n, None) is f for n, f in _BASIS))
 
     def _advect_rhs(self, data, deriv, scalar):
         """The whole right-hand side in one library call, in the reference's
@@ -338,3 +345,13 @@ class ReferenceOrderRHS:
             self.curlX(mathvector, deriv['B'])
         if self._shear:
             kaxpy(kval(deriv['B']['x']), kval(data['B']['y']), S, True)
+
+
+# What dd_advect_rhs3d replaces: the operators of the sequence and the
+# representation's part in them.
+_OPERATORS = [(n, getattr(ReferenceOrderRHS, n)) for n in
+              ('_aux', '_base_rhs', 'divX', 'XgradY', 'XconstcrossY', 'laplace_solve', 'pressure_projection',
+               '_generic_hydro')]
+_BASIS = [(n, getattr(FourierRepresentation, n)) for n in
+          ('_setup_k', 'set_fft', 'fwd_cuda', 'rev_cuda', 'forward', 'backward', 'require_space', 'dealias', 'deriv', 'k2',
+           '__getitem__', '__setitem__')]
