@@ -93,6 +93,7 @@ SIGNATURES = {
     "dd_xspace_fma": [I64, P, P, D, I, P, P],
     "dd_advect_workspace_size": [P, I, ctypes.POINTER(SZ)],
     "dd_advect_rhs3d": [P, I, P, P, PP, PP, P, SZ, P],
+    "dd_advect_rhs3d_aux": [P, I, P, P, PP, PP, PP, P, SZ, P],
     "dd_les_workspace_size": [P, I, ctypes.POINTER(SZ)],
     "dd_les_rhs3d": [P, PP, PP, P, I, I, P, P, SZ, P],
     "dd_les_rk4_step3d": [P, PP, P, PP, PP, P, I, D, I, ctypes.POINTER(I), P, P, SZ, P],

@@ -56,6 +56,8 @@ struct AdvArgs {
     CPtrs adv;              // (u.grad) Y, compact
     CPtrs y;                // u, T
     Ptrs d;                 // du, dT
+    double2* ms;            // work fields of the operator sequence as it leaves them, or null
+    double2* mv[3];
     int rotation, ns, dir;
     double om[3], gg, alpha_t, beta;
 };
@@ -63,6 +65,9 @@ struct AdvArgs {
 // All modes of the full layout, one per thread, bound by the FP64 pipe.  128-thread
 // blocks: 64^3 is 6.9 per SM, where 3.5 of 256 threads leave half a wave idle (27 us
 // at 64^3; 31 with those and a predicated buoyancy addition per axis).
+// a.ms, a.mv: what the sequence leaves in its work fields.  Without a scalar the
+// pressure term and Omega x u (without rotation the kept u), with one
+// beta u_dir and the kept u.
 __global__ void __launch_bounds__(128) k_advect_tail3(AdvArgs a) {
     grid_wait();
     const Geo3& g = a.g;
@@ -95,7 +100,12 @@ __global__ void __launch_bounds__(128) k_advect_tail3(AdvArgs a) {
                 const double2 m = make_double2(radd(rmul(u[q].x, a.om[p]), rmul(u[p].x, -a.om[q])),
                                                radd(rmul(u[q].y, a.om[p]), rmul(u[p].y, -a.om[q])));
                 N[c] = make_double2(radd(N[c].x, rmul(m.x, -2.)), radd(N[c].y, rmul(m.y, -2.)));
+                if (a.ms && a.ns == 3) a.mv[c][i] = m;
             }
+        }
+        if (a.ms && (a.ns == 4 || !a.rotation)) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) a.mv[c][i] = kept ? u[c] : make_double2(0., 0.);
         }
         if (a.ns == 4) {        // physics.py:688-708
             const double2 T = ((const double2*)a.y.p[3])[i];
@@ -107,7 +117,9 @@ __global__ void __launch_bounds__(128) k_advect_tail3(AdvArgs a) {
             if (a.dir == 0) N[0] = nd;
             else if (a.dir == 1) N[1] = nd;
             else N[2] = nd;
-            ((double2*)a.d.p[3])[i] = make_double2(rsub(N[3].x, rmul(ud.x, a.beta)), rsub(N[3].y, rmul(ud.y, a.beta)));
+            const double2 bu = make_double2(rmul(ud.x, a.beta), rmul(ud.y, a.beta));
+            ((double2*)a.d.p[3])[i] = make_double2(rsub(N[3].x, bu.x), rsub(N[3].y, bu.y));
+            if (a.ms) a.ms[i] = bu;
         }
         // pressure projection (physics.py:588-599, 407-416)
         const double kxv = a.kx[ix], kyv = a.ky[ky_i], kzv = a.kz[kz_i];
@@ -116,6 +128,7 @@ __global__ void __launch_bounds__(128) k_advect_tail3(AdvArgs a) {
         const double2 dx = ideriv(N[0], kxv), dy = ideriv(N[1], kyv), dz = ideriv(N[2], kzv);
         const double2 dv = make_double2(radd(radd(dx.x, dy.x), dz.x), radd(radd(dx.y, dy.y), dz.y));
         const double2 ph = make_double2(-rmul(dv.x, s), -rmul(dv.y, s));
+        if (a.ms && a.ns == 3) a.ms[i] = ph;
         const double2 gr[3] = {ideriv(ph, kxv), ideriv(ph, kyv), ideriv(ph, kzv)};
 #pragma unroll
         for (int c = 0; c < 3; c++)
@@ -174,8 +187,8 @@ int dd_advect_workspace_size(const dd_plan* p, int nscalar, size_t* bytes) {
     return DD_OK;
 }
 
-int dd_advect_rhs3d(const dd_plan* p, int nscalar, const double* omega, const double* params, const void* const* state,
-                    void* const* deriv, void* work, size_t work_bytes, void* stream) {
+int dd_advect_rhs3d_aux(const dd_plan* p, int nscalar, const double* omega, const double* params, const void* const* state,
+                        void* const* deriv, void* const* aux, void* work, size_t work_bytes, void* stream) {
     DD_CHECK_ARG(p && state && deriv && work, "dd_advect_rhs3d: null pointer");
     DD_CHECK_SUPPORTED(p->ndim == 3, "dd_advect_rhs3d: the plan must be 3D");
     DD_CHECK_ARG(nscalar == 0 || nscalar == 1, "dd_advect_rhs3d: nscalar must be 0 or 1");
@@ -196,8 +209,18 @@ int dd_advect_rhs3d(const dd_plan* p, int nscalar, const double* omega, const do
         a.y.p[c] = state[c];
         a.d.p[c] = deriv[c];
     }
+    if (aux) {
+        for (int c = 0; c < 4; c++) DD_CHECK_ARG(aux[c], "dd_advect_rhs3d: null work field %d", c);
+        a.ms = (double2*)aux[0];
+        for (int c = 0; c < 3; c++) a.mv[c] = (double2*)aux[1 + c];
+    }
     const cudaStream_t st = (cudaStream_t)stream;
     return nscalar ? advect_rhs3d<4>(p, a, work, work_bytes, st) : advect_rhs3d<3>(p, a, work, work_bytes, st);
+}
+
+int dd_advect_rhs3d(const dd_plan* p, int nscalar, const double* omega, const double* params, const void* const* state,
+                    void* const* deriv, void* work, size_t work_bytes, void* stream) {
+    return dd_advect_rhs3d_aux(p, nscalar, omega, params, state, deriv, nullptr, work, work_bytes, stream);
 }
 
 }  // extern "C"

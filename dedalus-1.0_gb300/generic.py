@@ -76,12 +76,38 @@ class ReferenceOrderRHS:
     laplace_k2 = 'cached'
 
     # ---------------------------------------------------------- helpers
+    # aux_fields (physics.py:108-119): created by the first right-hand side of the
+    # operator sequence.  One-call right-hand sides leave their values in plain arrays
+    # (time, [k arrays]) until somebody asks for the fields: the fields' host
+    # tables take longer than a whole 64^3 step.
+    _aux_state = None
+    _aux_work = None
+
+    @property
+    def aux_fields(self):
+        if self._aux_state is None and self._aux_work is None:
+            raise AttributeError("aux_fields exist after a right-hand side of the operator sequence")
+        return self._aux()
+
+    @aux_fields.setter
+    def aux_fields(self, fields):
+        self._aux_state = fields
+
     def _aux(self):
-        aux = getattr(self, 'aux_fields', None)
-        if aux is None:
-            # physics.py:108-113, 118-119
-            aux = self.aux_fields = self.create_fields(0., self._aux_field_list)
-        return aux
+        if self._aux_state is None:
+            self._aux_state = self.create_fields(0., self._aux_field_list)
+            if self._aux_work is not None:
+                time, arrays = self._aux_work
+                self._aux_work = None
+                self._aux_state.set_time(time)
+                for c, k in zip(self._advect_work(), arrays):
+                    c.kdata = k
+                    _kset(c)
+        return self._aux_state
+
+    def _advect_work(self):
+        """Components of the work fields that the one-call right-hand sides write."""
+        return [self._aux_state['mathscalar'].components[0]] + [self._aux_state['mathvector'][i] for i in range(3)]
 
     def _base_rhs(self, data, deriv):
         # physics.py:134-149
@@ -238,9 +264,14 @@ class ReferenceOrderRHS:
 
     def _advect_rhs(self, data, deriv, scalar):
         """The whole right-hand side in one library call, in the reference's
-        operator order and roundings (generic operator sequence below)."""
+        operator order and roundings (generic operator sequence below).  The work
+        fields (aux_fields) are left as the sequence leaves them, the vector of a
+        Boussinesq one in k-space."""
         self._generic_if(deriv)
         deriv.set_time(data.time)
+        for fname, field in deriv:
+            if fname not in ('u', 'T') or (fname == 'T' and not scalar):
+                field.zero_all()
         comps = [data['u'][i] for i in range(3)] + ([data['T'].components[0]] if scalar else [])
         outs = [deriv['u'][i] for i in range(3)] + ([deriv['T'].components[0]] if scalar else [])
         plan = self.plan(data)
@@ -257,7 +288,19 @@ class ReferenceOrderRHS:
         ws = self.workspace(n.value)
         sp, _a = _lib.ptr_array([kval(c).data_ptr() for c in comps])
         dp, _b = _lib.ptr_array([c.kdata.data_ptr() for c in outs])
-        _lib.call("dd_advect_rhs3d", plan.handle, int(scalar), om, params, sp, dp, dptr(ws), ws.numel(),
+        if self._aux_state is None:
+            work = self._aux_work[1] if self._aux_work else [torch.empty_like(outs[0].kdata) for _ in range(4)]
+            self._aux_work = (data.time, work)
+        else:
+            self._aux_state.set_time(data.time)
+            for fname, field in self._aux_state:
+                if fname not in ('mathscalar', 'mathvector'):
+                    field.zero_all()
+            for c in self._advect_work():
+                _kset(c)
+            work = [c.kdata for c in self._advect_work()]
+        wp, _c = _lib.ptr_array([t.data_ptr() for t in work])
+        _lib.call("dd_advect_rhs3d_aux", plan.handle, int(scalar), om, params, sp, dp, wp, dptr(ws), ws.numel(),
                   current_stream())
         for c in outs:
             _kset(c)

@@ -414,6 +414,13 @@ int dd_xspace_fma(int64_t n, const double* a, const double* b, double w, int acc
 int dd_advect_workspace_size(const dd_plan* plan, int nscalar, size_t* bytes);
 int dd_advect_rhs3d(const dd_plan* plan, int nscalar, const double* omega, const double* params,
                     const void* const* state, void* const* deriv, void* work, size_t work_bytes, void* stream);
+/* The same, and aux (NULL or four full-layout k arrays: a scalar, then x, y, z of a
+ * vector) gets what the reference's operators leave in their work fields
+ * mathscalar and mathvector: with nscalar = 0 the pressure term and Omega x u
+ * (without rotation the dealiased u), with nscalar = 1 beta u_dir and the dealiased u. */
+int dd_advect_rhs3d_aux(const dd_plan* plan, int nscalar, const double* omega, const double* params,
+                        const void* const* state, void* const* deriv, void* const* aux, void* work, size_t work_bytes,
+                        void* stream);
 
 #ifdef __cplusplus
 }
