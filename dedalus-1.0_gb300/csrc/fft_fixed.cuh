@@ -23,9 +23,9 @@
 // that both pipes work; on the way out everything is integer.
 //
 // Values below 2^-62 of the bound vanish, as they do in an FP64 sum with the
-// larger ones.  A pencil whose largest value is outside 2^-895 .. 2^49 is
-// scaled by 2^512 or 2^-975 on the way in and back on the way out.  One that holds a NaN or an
-// infinity gives NaN everywhere.
+// larger ones.  A pencil whose largest value is outside 2^-895 .. 2^49, subnormal
+// ones included, is scaled by 2^512 or 2^-975 on the way in and back on the way out.
+// One that holds a NaN or an infinity gives NaN everywhere.
 #pragma once
 #include <type_traits>
 
@@ -36,7 +36,7 @@ namespace dd {
 typedef long long fx;      // one fixed-point value
 
 // --------------------------------------------------- scales
-// 1 - largest |x| high word of a pencil (0 = all zero) to its bound: every
+// 1 - largest |x| high word of a pencil (0 = zeros and subnormals) to its bound: every
 // component is below 2^(e2 - 1022.5), a pair's modulus below 2^(e2 - 1022).
 // rare: 0, or 1 (times 2^512 on the way in), 2 (times 2^-975), 3 (not finite).
 struct FxScale {
@@ -48,8 +48,7 @@ __host__ __device__ __forceinline__ FxScale fx_scale(unsigned m) {
     // exponent of sqrt(2) (m + 1): carries where the 20 mantissa bits exceed sqrt(2) - 1
     s.e2 = (int)((m + 614242u) >> 20);
     s.rare = 0;
-    if (m == 0u) s.e2 = 1023;
-    else if (m >= 0x7ff00000u) { s.rare = 3; s.e2 = 1023; }
+    if (m >= 0x7ff00000u) { s.rare = 3; s.e2 = 1023; }
     else if (s.e2 < 128) { s.rare = 1; s.e2 = (s.e2 > 1 ? s.e2 : 1) + 512; }
     else if (s.e2 > 1072) { s.rare = 2; s.e2 -= 975; }
     return s;
@@ -63,9 +62,16 @@ __device__ __forceinline__ double fx_post(int rare) {
 
 // v[i] *= f behind a branch: FP64 instructions take 64 clocks of their pipe
 // per warp even where a predicate turns them off, and a branch around each
-// single one becomes such a predicate.
+// single one becomes such a predicate.  Zeros skip it: pencils of zeros are
+// among the pre-scaled ones.
 template <int N>
 __device__ __forceinline__ void fx_scale_all(C<double>* v, double f) {
+    unsigned nz = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        nz |= (unsigned)__double2hiint(v[i].x) | (unsigned)__double2loint(v[i].x) | (unsigned)__double2hiint(v[i].y) |
+              (unsigned)__double2loint(v[i].y);
+    if (nz == 0u) return;
 #pragma unroll
     for (int i = 0; i < N; i++) { v[i].x *= f; v[i].y *= f; }
 }
@@ -445,7 +451,7 @@ __device__ __forceinline__ void fx_finish(C<double>* tile, const C<fx> (&v)[fx_b
 }
 
 // Transform S::P pencils (thread: pencil p, butterflies jt + b TPP).  smax:
-// FX_WORDS arrays of P shared words, zero on entry.  The caller synchronises
+// FX_WORDS arrays of P shared words, zero on entry (the first may hold a high word already).  The caller synchronises
 // before, except that FX_IN_GLOBAL does so itself once its loads are issued
 // (staged twiddles and cleared maxima become visible there); FX_OUT_TILE returns
 // synchronised.  PRUNE as in pencil_fft_s: inputs of the removed band are taken
