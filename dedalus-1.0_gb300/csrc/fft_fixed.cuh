@@ -534,9 +534,13 @@ template <int L, bool INV, int P, class CC = FxCfg<L>>
 using FxR = Sched<L, P, P * FxRowTPP<L>::v, INV ? CC::R[0] : CC::RF[0], INV ? CC::R[1] : CC::RF[1],
                   INV ? CC::R[2] : CC::RF[2], (P | 1), 1>;
 
-// Shared words of a block of P groups of two warps (three reductions).
+// Shared words of a block of P groups of two warps (three reductions).  Such groups
+// synchronise on the named barriers 1 to 15, one each.
 template <class S>
-constexpr int fx_group_words() { return S::TPP > 32 ? 6 * S::P : 0; }
+constexpr int fx_group_words() {
+    static_assert(S::TPP <= 32 || S::P <= 15, "more groups of two warps than named barriers");
+    return S::TPP > 32 ? 6 * S::P : 0;
+}
 
 template <int TPP>
 __device__ __forceinline__ unsigned fx_group_mask() {
