@@ -147,7 +147,7 @@ __device__ __forceinline__ fx fx_shl(fx a, int n) {       // 0 <= n < 32
 
 // a (c + i s) / 2^(2 + n) for a twiddle c + i s = (w.x 2^32 + w.y + i (w.z 2^32 + w.w)) 2^-62
 // (signed halves), half = 2^(31 + n): rounded to nearest up to the product of
-// the low halves (below one unit before the division).  |a| < 2^62, n <= 2.
+// the low halves (below one unit before the division).  |a| < 2^62, n <= 1.
 __device__ __forceinline__ C<fx> fx_twiddle(C<fx> a, int4 w, int n, fx half) {
     const FxHL x = fx_split(a.x), y = fx_split(a.y);
     fx re = fx_mad(x.h, w.y, half), im = fx_mad(x.h, w.w, half);
@@ -176,44 +176,17 @@ __device__ __forceinline__ fx fx_mul63(fx a, int ch, int cl) {
 #define DD_FX_R2L (-51432894)
 #define DD_FX_S3H 1859775393
 #define DD_FX_S3L 1630710223
-// cos and sin of pi/8 in units of 2^-62
-#define DD_FX_C8H 992008094
-#define DD_FX_C8L 1696238673
-#define DD_FX_S8H 410903207
-#define DD_FX_S8L (-1364630830)
 
-// a W_16^M (forward) or its conjugate (inverse), M a compile-time constant;
-// |a| < 2^60 (odd M) or 2^61.
+// a W_8^M (forward) or its conjugate (inverse), M = 1 or 3; |a| < 2^61.
 template <int M, bool INV>
-__device__ __forceinline__ C<fx> fx_rot16(C<fx> a) {
-    constexpr int m = M % 16;
-    if constexpr (m == 0) {
-        return a;
-    } else if constexpr (m == 4) {
-        return mul_mi<INV>(a);
-    } else if constexpr (m == 2) {             // (1 -+ i) / sqrt 2
+__device__ __forceinline__ C<fx> fx_rot8(C<fx> a) {
+    static_assert(M == 1 || M == 3, "rotations of the radix-8 butterfly");
+    if constexpr (M == 1) {                    // (1 -+ i) / sqrt 2
         const fx p = fx_mul63(a.x + a.y, DD_FX_R2H, DD_FX_R2L), d = fx_mul63(a.y - a.x, DD_FX_R2H, DD_FX_R2L);
         return INV ? mk<fx>(-d, p) : mk<fx>(p, d);
-    } else if constexpr (m == 6) {             // (-1 -+ i) / sqrt 2
+    } else {                                   // (-1 -+ i) / sqrt 2
         const fx p = fx_mul63(a.x + a.y, DD_FX_R2H, DD_FX_R2L), d = fx_mul63(a.y - a.x, DD_FX_R2H, DD_FX_R2L);
         return INV ? mk<fx>(-p, -d) : mk<fx>(d, -p);
-    } else {
-        static_assert(m == 1 || m == 3 || m == 9, "unused rotation");
-        // 4 a.h fits 32 bits
-        constexpr bool swap = m == 3;
-        constexpr int sg = m == 9 ? -1 : 1;    // W^9 = -W^1
-        constexpr int ch = sg * (swap ? DD_FX_S8H : DD_FX_C8H), cl = sg * (swap ? DD_FX_S8L : DD_FX_C8L);
-        constexpr int s0h = sg * (swap ? DD_FX_C8H : DD_FX_S8H), s0l = sg * (swap ? DD_FX_C8L : DD_FX_S8L);
-        constexpr int sh = INV ? s0h : -s0h, sl = INV ? s0l : -s0l;
-        const FxHL x = fx_split(a.x), y = fx_split(a.y);
-        const fx half = 1ll << 29;
-        fx re = fx_mad(x.l, ch, fx_mad(x.h, cl, half)), im = fx_mad(x.l, sh, fx_mad(x.h, sl, half));
-        re = fx_mad(y.l, -sh, fx_mad(y.h, -sl, re)) >> 30;
-        im = fx_mad(y.l, ch, fx_mad(y.h, cl, im)) >> 30;
-        const int x4 = 4 * x.h, y4 = 4 * y.h;
-        re = fx_mad(y4, -sh, fx_mad(x4, ch, re));
-        im = fx_mad(y4, ch, fx_mad(x4, sh, im));
-        return mk<fx>(re, im);
     }
 }
 
@@ -227,35 +200,13 @@ __device__ __forceinline__ void fx_dft(C<fx>* v) {
         C<fx> o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
         dft4<INV>(e0, e1, e2, e3);
         dft4<INV>(o0, o1, o2, o3);
-        o1 = fx_rot16<2, INV>(o1);
-        o2 = fx_rot16<4, INV>(o2);
-        o3 = fx_rot16<6, INV>(o3);
+        o1 = fx_rot8<1, INV>(o1);
+        o2 = mul_mi<INV>(o2);
+        o3 = fx_rot8<3, INV>(o3);
         v[0] = e0 + o0; v[4] = e0 - o0;
         v[1] = e1 + o1; v[5] = e1 - o1;
         v[2] = e2 + o2; v[6] = e2 - o2;
         v[3] = e3 + o3; v[7] = e3 - o3;
-    } else if constexpr (R == 16) {
-        C<fx> y[4][4];
-#pragma unroll
-        for (int n2 = 0; n2 < 4; n2++) {
-            y[n2][0] = v[n2]; y[n2][1] = v[4 + n2]; y[n2][2] = v[8 + n2]; y[n2][3] = v[12 + n2];
-            dft4<INV>(y[n2][0], y[n2][1], y[n2][2], y[n2][3]);
-        }
-        y[1][1] = fx_rot16<1, INV>(y[1][1]);
-        y[1][2] = fx_rot16<2, INV>(y[1][2]);
-        y[1][3] = fx_rot16<3, INV>(y[1][3]);
-        y[2][1] = fx_rot16<2, INV>(y[2][1]);
-        y[2][2] = fx_rot16<4, INV>(y[2][2]);
-        y[2][3] = fx_rot16<6, INV>(y[2][3]);
-        y[3][1] = fx_rot16<3, INV>(y[3][1]);
-        y[3][2] = fx_rot16<6, INV>(y[3][2]);
-        y[3][3] = fx_rot16<9, INV>(y[3][3]);
-#pragma unroll
-        for (int k1 = 0; k1 < 4; k1++) {
-            C<fx> a0 = y[0][k1], a1 = y[1][k1], a2 = y[2][k1], a3 = y[3][k1];
-            dft4<INV>(a0, a1, a2, a3);
-            v[k1] = a0; v[k1 + 4] = a1; v[k1 + 8] = a2; v[k1 + 12] = a3;
-        }
     } else {
         static_assert(R == 3, "unsupported radix");
         const C<fx> t1 = v[1] + v[2], r = mul_mi<INV>(v[1] - v[2]);
@@ -297,7 +248,7 @@ template <int L, bool INV, int P = FxCfg<L>::P, class CC = FxCfg<L>>
 using FxS = Sched<L, P, P * CC::TPP, INV ? CC::R[0] : CC::RF[0], INV ? CC::R[1] : CC::RF[1], INV ? CC::R[2] : CC::RF[2]>;
 
 // Bits of growth of a pass: log2 R, and 2 for R = 3.
-constexpr int fx_bits(int R) { return R == 16 ? 4 : R == 8 ? 3 : 2; }
+constexpr int fx_bits(int R) { return R == 8 ? 3 : 2; }
 
 // Radix-R butterflies per thread of a pencil's TPP threads: j = jt + b TPP for
 // those with fx_has.
@@ -321,7 +272,7 @@ __device__ __forceinline__ int fx_row(int base, int r) {
 // K of fx_in for a pencil of bound e2 (packed: of sums of two such values).
 template <class S>
 __host__ __device__ constexpr int fx_kin(int e2, bool packed) {
-    static_assert(S::R1 == 4 || S::R1 == 8 || S::R1 == 16, "first radix");
+    static_assert(S::R1 == 4 || S::R1 == 8, "first radix");
     return e2 + 1 + fx_bits(S::R1) + (packed ? 1 : 0);
 }
 
