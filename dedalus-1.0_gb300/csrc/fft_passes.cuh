@@ -279,7 +279,12 @@ int launch_pass_small(int L, const Op& op, int npencil, int nslow, int nfield, c
 // grids, chosen per plan by the ensemble autotuner (dd_plan_set_schedule):
 // the same radix sequence as the default (so every pencil's arithmetic, and
 // its result, is identical) on fewer pencils per block: variant 1 the
-// smallest tile (2-4 pencils), variant 2 a middle one (4-8 pencils).
+// smallest tile (2-4 pencils), variant 2 a middle one (4-8 pencils).  The FP64
+// default has 8 pencils itself, so that at 64 and 128 points variant 2 is the
+// default; 2 pencils in its place are never faster than 4 and slower for many
+// runs (a step of 64 runs of 128^2 240 us, 217 with 4 or 8 pencils).  A single run's
+// default is a small tile already (SmallSched): at 256 and 512 points FP64 variant 1.
+// The ensemble autotuner leaves these equal ones out.
 constexpr int kYSchedVariants = 3;
 template <int L, int V> struct YVariant;
 template <> struct YVariant<64, 1>  { using S = Sched<64, 4, 32, 8, 8, 1>; };

@@ -11,8 +11,8 @@ classes are issued on their own CUDA streams, and a complete ensemble step
 an ensemble step costs one graph launch on the host.
 
 ``autotune`` measures, per size class, the tile schedule of its y passes
-(dd_plan_set_schedule: the default tile or two smaller ones with the same
-radix sequence, so results are bitwise unchanged for classes of more than
+(dd_plan_set_schedule: the default tile or up to two smaller ones with the
+same radix sequence, so results are bitwise unchanged for classes of more than
 one run), the chunking of its runs
 (runs per launch) and the order in which classes are issued, keeps the
 fastest schedule and caches it in a JSON file keyed by GPU, size, run count
@@ -71,6 +71,17 @@ class _SizeClass:
         v, n = ctypes.c_int(), ctypes.c_int()
         _lib.call("dd_plan_get_schedule", self.plan.handle, 0, ctypes.byref(v), ctypes.byref(n))
         return n.value
+
+    def yscheds(self):
+        """The tile variants worth timing: without the FP64 ones that are the default tile
+        itself (dd_plan_set_schedule in dd_gb300.h)."""
+        v = list(range(self.ysched_count()))
+        if self.precision == _lib.DD_FP64 and len(v) > 1:
+            if self.nrun > 1 and self.n <= 128:
+                v.remove(2)
+            elif self.nrun == 1 and self.n >= 256:
+                v.remove(1)
+        return v
 
     def workspace(self, chunk):
         n = ctypes.c_size_t()
@@ -322,7 +333,7 @@ class BoussinesqEnsemble2D:
         best = self._time_schedule(dt)
         for c in self.classes:
             best_ys = c.ysched
-            for ys in range(c.ysched_count()):
+            for ys in c.yscheds():
                 if ys == best_ys:
                     continue
                 c.set_ysched(ys)

@@ -77,11 +77,14 @@ int dd_plan_destroy(dd_plan* plan);
 
 /* Tile schedule of a pass group of this plan (which = 0: the y passes of the
  * fused 2D steps, dd_rhs2d / dd_rk2mid_step2d): variant 0 is the default,
- * 1 and 2 run the default tile's radix sequence on smaller tiles (bitwise the
- * same results, except against a single run of 64 or 128 points, whose
- * default is the small-tile schedule with its own radix sequence); dd_plan_get_schedule reports the current variant and how many this
- * plan's length offers (3 for 64, 128, 256, 512 points, else 1; a variant
- * the length lacks runs the default).  Set by the ensemble autotuner.  No
+ * 1 and 2 run the default tile's radix sequence on tiles of 2-4 and 4-8 pencils
+ * (bitwise the same results, except against a single run of 64 or 128 points, whose
+ * default is the small-tile schedule with its own radix sequence).  For several
+ * runs the default tile is wider (8 pencils or more), but in FP64 at 64 and 128 points
+ * variant 2 is the default tile; for a single run the default has 4 (64 and 128
+ * points) or 2 pencils (256 and 512).  dd_plan_get_schedule reports the current
+ * variant and how many this plan's length offers (3 for 64, 128, 256, 512 points, else
+ * 1; a variant the length lacks runs the default).  Set by the ensemble autotuner.  No
  * counterpart in the reference (FFTW chooses its own plans:
  * dedalus/utils/fftw/_fftw.pyx:246-309, flags FFTW_MEASURE). */
 int dd_plan_set_schedule(dd_plan* plan, int which, int variant);
