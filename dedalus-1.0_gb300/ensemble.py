@@ -15,8 +15,8 @@ an ensemble step costs one graph launch on the host.
 same radix sequence, so results are bitwise unchanged for classes of more than
 one run), the chunking of its runs
 (runs per launch) and the order in which classes are issued, keeps the
-fastest schedule and caches it in a JSON file keyed by GPU, size, run count
-and precision.  Each size class owns its plan, so a tuned schedule does not
+fastest schedule and caches it in a JSON file keyed by GPU, size, run count,
+precision and SCHEDULE_REV.  Each size class owns its plan, so a tuned schedule does not
 leak into other users of the same grid size.
 """
 import ctypes
@@ -39,6 +39,9 @@ DIV_TOL2 = 1e-24
 # to 1e-6, below the FP32 path's own error, still takes the divergence form.
 DIV_TOL2_FP32 = 1e-12
 _TUNE_ENV = "DD_TUNE_CACHE"
+# Part of the key of cached schedules: raised whenever the 2D passes change enough
+# for choices timed before to be stale (2: fixed-point FP64 transforms).
+SCHEDULE_REV = 2
 
 
 def _default_cache():
@@ -311,8 +314,8 @@ class BoussinesqEnsemble2D:
         JSON.  Returns the schedule."""
         cache = cache or _default_cache()
         gpu = torch.cuda.get_device_name(self.device)
-        key = "%s|%s|%s|%s" % (gpu, self.precision, ",".join(str(c.n) for c in self.classes),
-                               ",".join(str(c.nrun) for c in self.classes))
+        key = "%s|%s|%s|%s|r%d" % (gpu, self.precision, ",".join(str(c.n) for c in self.classes),
+                                   ",".join(str(c.nrun) for c in self.classes), SCHEDULE_REV)
         db = {}
         if os.path.isfile(cache):
             try:
