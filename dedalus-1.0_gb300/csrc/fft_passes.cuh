@@ -253,7 +253,10 @@ int launch_pass(const Op& op, int npencil, int nslow, int nfield, cudaStream_t s
 // Small-tile schedules for single-run 2D grids: 4 pencils of 16 threads, and at
 // 256 and 512 points 2 pencils of the usual threads and radices (a 512-point y pass of
 // 171 kx pencils of 3 fields is 66 tiles of 8, or 258 of 2, for 152 SMs: a 512^2
-// convection step takes 181 us, 195 with 8; a 512^2 hydro step 138, 146 with 8).
+// convection step takes 181 us, 195 with 8; a 512^2 hydro step 138, 146 with 8).  The
+// lengths 48, 96 and 192 keep the wide tiles: graphs of single steps of 48^2, 96^2 and
+// 192^2 take 794, 813 and 816 us in FP64 (most of it phi functions without tables), 793,
+// 811 and 812 with tiles of 4, 2 and 2, but 807, 832 and 837 against 800, 820 and 837 in FP32.
 template <typename T, int L, bool INV> struct SmallSched { using S = Sched<L, 2, 2 * DefSched<L>::TPP, DefSched<L>::R1, DefSched<L>::R2, DefSched<L>::R3>; };
 template <int L, bool INV> struct SmallSched<double, L, INV> { using S = FxS<L, INV, 2>; };
 template <typename T, bool INV> struct SmallSched<T, 64, INV> { using S = Sched<64, 4, 64, 4, 4, 4>; };

@@ -71,11 +71,11 @@ __global__ void k_stage2(Stage2Args a) {
     const Geo2& g = a.g;
     const int per = g.Kx * g.Ky;
     const int64_t n = (int64_t)per * a.nrun;
-    // The kernel is bound by the FP64 pipe.  With integer wavenumbers and their q
-    // tables k^2 is an integer below 2^24, exact in float; the RK stages (MODE > 0)
+    // The kernel is bound by the FP64 pipe.  Callers give q tables for integer
+    // wavenumbers with k^2 below 2^24 only, exact in float; the RK stages (MODE > 0)
     // fuse multiplications into additions and share the phi functions of the two
     // velocity components: Boussinesq 49 -> 36 operations per mode in stage 1,
-    // 67 -> 49 in stage 2 (512-run ensemble step 9.38 -> 8.65 ms together with the group x passes).
+    // 67 -> 49 in stage 2 (128-run ensemble step 3015 -> 2885 us).
     bool tabs = a.intk && a.inv_k2;
     if constexpr (MODE != 0) {
 #pragma unroll

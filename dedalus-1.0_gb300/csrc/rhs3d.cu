@@ -168,7 +168,7 @@ __global__ void k_rk4_stage3(RK4Args a) {
     const Geo3& g = a.pa.g;
     constexpr int NF = Phys3<PH>::NF, NG = Phys3<PH>::NG;
     const int n = g.Ky * g.Kz * g.Kx;      // < 2^31 for every supported grid
-    // integer wavenumbers with their q tables: k^2 is an integer below 2^24,
+    // callers give q tables for integer wavenumbers with k^2 below 2^24 only,
     // exact in float (the kernel is bound by the FP64 pipe: 55 -> 49 operations
     // per mode of the hydro divergence form, 280 -> 252 us per launch at 256^3)
     const bool tabs = a.pa.intk && a.pa.inv_k2 && a.tab[0] && (NG == 1 || a.tab[1]);

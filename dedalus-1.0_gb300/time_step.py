@@ -9,9 +9,10 @@ dt=None)``, ``do_advance(data, dt)``, stop controls (``ok``,
 Two execution paths give the same result (to roundoff):
 * fused: one C-ABI call per step (RK4 for 3D hydro: ``dd_hydro3d_rk4_step``),
   chosen automatically when the physics provides it;
-* generic: ``RHS(data, deriv)`` plus the reference's stage kernels
-  (``dd_euler``/``dd_etd1``/``dd_etd2rk1``/``dd_etd2rk2``) on the device,
-  exactly as the reference sequences them.
+* generic: ``RHS(data, deriv)`` plus the reference's stage updates on the
+  device, as the reference sequences them: fields with an integrating factor in
+  one ``dd_etd_fields`` call per stage (RK2mid, RK2trap) or one ``dd_etd1`` each
+  (RK4), fields without one in ``dd_euler``.
 
 RK4 follows the project's definition of the reference's unrunnable RK4
 (``linear_step == euler``, ``intfac_step == etd1`` with ``-IF``, each stage's
