@@ -4,7 +4,8 @@ with ``shear_rate`` != 0), rotation (``Omega``), 3D Boussinesq and 2D MHD.
 Rotation and 3D Boussinesq without shear, on axes of 16 to 512 points, run as
 one library call with the same operand order (``dd_advect_rhs3d``,
 ``_advect_rhs``), unless a subclass or an instance has operators, a representation
-or a k^2 of its own (``_advect_fused``); everything else runs operator by operator.
+or a k^2 of its own (``_advect_fused``), or the derivative is the state itself (the
+sequence zeroes it first); everything else runs operator by operator.
 
 The operator helpers are the reference's (dedalus/physics/physics.py:
 ``divX`` 180-195, ``XgradY`` 197-228, ``XconstcrossY`` 266-307,
@@ -313,7 +314,7 @@ class ReferenceOrderRHS:
     def _generic_hydro(self, data, deriv, project):
         """IncompressibleHydro.RHS (physics.py:527-586); tracer and forcing are
         refused by _finalize."""
-        if project and self._advect_fused(data):
+        if project and deriv is not data and self._advect_fused(data):
             return self._advect_rhs(data, deriv, False)
         self._generic_if(deriv)
         self._base_rhs(data, deriv)
@@ -339,7 +340,7 @@ class ReferenceOrderRHS:
 
     def _generic_boussinesq(self, data, deriv):
         """BoussinesqHydro.RHS (physics.py:664-712)."""
-        if self._advect_fused(data):
+        if deriv is not data and self._advect_fused(data):
             return self._advect_rhs(data, deriv, True)
         self._generic_hydro(data, deriv, project=False)
         mathscalar = self.aux_fields['mathscalar']

@@ -58,3 +58,17 @@ def test_work_fields(dd, cuda, name, shape, params, looks):
             else:
                 assert np.array_equal(x, y), (f, i, space)
             assert np.any(y) == (f != "own")
+
+
+@pytest.mark.parametrize("name,shape,params", _CASES)
+def test_derivative_in_the_state_itself(dd, cuda, name, shape, params):
+    """RHS(data, data): the sequence zeroes the derivative, so the state, first (physics.py:140-142)."""
+    M = dd.mods
+    p = getattr(M, name)(shape, M.FourierRepresentation)
+    p.parameters.update(params)
+    d = p.create_fields(0.7)
+    for f, field in d:
+        for i, c in field:
+            c["xspace"] = np.random.default_rng(i).standard_normal(shape)
+    p.RHS(d, d)
+    assert not any(np.any(c.to_numpy("kspace")) for f, field in d for i, c in field)
