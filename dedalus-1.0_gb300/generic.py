@@ -77,6 +77,25 @@ class ReferenceOrderRHS:
     laplace_k2 = 'cached'
 
     # ---------------------------------------------------------- helpers
+    # k^2 of the pressure solve: None until laplace_solve has cached it or the user has
+    # set it.  After one-call right-hand sides, which use the plan's wavenumbers, it is
+    # made when somebody asks for it.
+    _k2 = None
+    _k2_seen = None
+    _advected = False
+
+    @property
+    def k2(self):
+        if self._k2 is None and self._advected and self.laplace_k2 != 'current':
+            if self._k2_seen is None:
+                self._k2_seen = self.aux_fields['mathscalar'].components[0].k2(no_zero=True)
+            return self._k2_seen
+        return self._k2
+
+    @k2.setter
+    def k2(self, k2):
+        self._k2 = k2
+
     # aux_fields (physics.py:108-119): created by the first right-hand side of the
     # operator sequence.  One-call right-hand sides leave their values in plain arrays
     # (time, [k arrays]) until somebody asks for the fields: the fields' host
@@ -255,11 +274,12 @@ class ReferenceOrderRHS:
     def _advect_fused(self, data):
         """True when dd_advect_rhs3d covers this 3D right-hand side: a static
         basis (no shear), axis lengths of the fused passes, and the operators, the
-        representation and k^2 that the call stands for (a k2 set on the object
-        before its first right-hand side is used by laplace_solve only)."""
+        representation and k^2 that the call stands for (a k2 that the user has set or
+        written to is used by laplace_solve only)."""
         return (self.ndim == 3 and not self._shear and self._representation._static_k
                 and min(self.plan(data).xshape) >= 16
-                and (self.k2 is None or self.laplace_k2 == 'current')
+                and (self.laplace_k2 == 'current' or
+                     (self._k2 is None and (self._k2_seen is None or self._k2_seen._version == 0)))
                 and all(getattr(getattr(self, n), '__func__', None) is f for n, f in _OPERATORS)
                 and all(getattr(self._representation, n, None) is f for n, f in _BASIS))
 
@@ -269,6 +289,7 @@ class ReferenceOrderRHS:
         fields (aux_fields) are left as the sequence leaves them, the vector of a
         Boussinesq one in k-space."""
         self._generic_if(deriv)
+        self._advected = True
         deriv.set_time(data.time)
         for fname, field in deriv:
             if fname not in ('u', 'T') or (fname == 'T' and not scalar):

@@ -104,3 +104,26 @@ def test_stock_classes_take_one_call(dd, cuda, base):
         assert p._advect_fused(d)
         p.RHS(d, o)
         assert p._advect_fused(d)
+
+
+@pytest.mark.parametrize("base", list(PARAMS))
+def test_k2_after_a_right_hand_side(dd, cuda, base):
+    """The k^2 that laplace_solve caches at the first call is there, reading it changes nothing, and
+    writing to it, in place or not, reaches the pressure solve."""
+    p, s = _make(dd, base), _make(dd, base)
+    s._advect_fused = lambda data: False
+    assert p.k2 is None and s.k2 is None
+    k = _state()
+    first = _rhs(p, k)
+    _rhs(s, k)
+    assert np.array_equal(p.k2.cpu().numpy(), s.k2.cpu().numpy()) and p.k2 is p.k2
+    assert p._advect_fused(p.create_fields(0.))
+    assert all(np.array_equal(x, y) for x, y in zip(_rhs(p, k), first))
+    for change in (lambda q: q.k2.add_(3.0), lambda q: setattr(q, "k2", q.k2 * 2.0)):
+        change(p)
+        change(s)
+        assert all(np.array_equal(x, y) for x, y in zip(_rhs(p, k), _rhs(s, k)))
+    p = _make(dd, base)
+    p.laplace_k2 = "current"
+    _rhs(p, k)
+    assert p.k2 is None
